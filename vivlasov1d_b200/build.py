@@ -10,6 +10,8 @@ from __future__ import annotations
 import os
 import subprocess
 import sys
+import tempfile
+from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
@@ -17,8 +19,9 @@ CSRC = os.path.join(HERE, "csrc")
 INCLUDE = os.path.join(ROOT, "include")
 LIB = os.path.join(HERE, "libvv.so")
 
-SOURCES = ["vv_api.cu", "vv_noalloc.cu"]
-HEADERS = ["vv_common.cuh", "vv_bracket.cuh", "vv_pc.cuh", "vv_pcj.cuh", "vv_pcv.cuh", "vv_coll.cuh", "vv_vec.cuh", "vv_batch.cuh", "vv_adjoint.cuh", "vv_pred.cuh"]
+SOURCES = ["vv_api.cu", "vv_noalloc.cu", "vv_cluster.cu"]
+HEADERS = ["vv_common.cuh", "vv_bracket.cuh", "vv_pc.cuh", "vv_pcj.cuh", "vv_pcv.cuh", "vv_coll.cuh", "vv_vec.cuh", "vv_batch.cuh", "vv_adjoint.cuh", "vv_pred.cuh",
+           "vv_cluster.h", "vv_cluster.cuh"]
 
 NVCC_FLAGS = [
     "-O3", "-std=c++17",
@@ -45,16 +48,22 @@ def build_library(force=False, verbose=False):
     deps = [os.path.join(CSRC, s) for s in SOURCES + HEADERS] + [os.path.join(INCLUDE, "vv.h")]
     if not force and not _stale(LIB, deps):
         return LIB
-    cmd = [nvcc()] + NVCC_FLAGS + ["-I", INCLUDE, "-I", CSRC, "-shared", "-o", LIB + ".tmp"]
-    if verbose:
-        cmd += ["-Xptxas", "-v"]
-    cmd += [os.path.join(CSRC, s) for s in SOURCES]
-    proc = subprocess.run(cmd, capture_output=True, text=True)
-    if proc.returncode != 0:
-        sys.stderr.write(proc.stdout + proc.stderr)
-        raise RuntimeError("nvcc failed building libvv.so")
-    if verbose:
-        sys.stderr.write(proc.stderr)
+    base = [nvcc()] + NVCC_FLAGS + ["-I", INCLUDE, "-I", CSRC] + (["-Xptxas", "-v"] if verbose else [])
+
+    def run(cmd):
+        proc = subprocess.run(cmd, capture_output=True, text=True)
+        if proc.returncode != 0:
+            sys.stderr.write(proc.stdout + proc.stderr)
+            raise RuntimeError("nvcc failed building libvv.so")
+        if verbose:
+            sys.stderr.write(proc.stderr)
+
+    # one object per source, compiled side by side
+    with tempfile.TemporaryDirectory() as tmp:
+        objs = [os.path.join(tmp, s + ".o") for s in SOURCES]
+        with ThreadPoolExecutor() as pool:
+            list(pool.map(run, [base + ["-c", os.path.join(CSRC, s), "-o", o] for s, o in zip(SOURCES, objs)]))
+        run(base + ["-shared", "-o", LIB + ".tmp"] + objs)
     os.replace(LIB + ".tmp", LIB)
     return LIB
 

@@ -17,6 +17,8 @@
 #include "vv_pcv.cuh"
 #include "vv_coll.cuh"
 #include "vv_pred.cuh"
+#include "vv_cluster.h"
+#include "vv_cluster.cuh"
 
 #include <algorithm>
 #include <array>
@@ -129,6 +131,16 @@ struct vv_ctx {
     // discrete adjoint (allocated at the first adjoint call): GMRES operator
     // switch, coefficient planes of J_H^T and J_Fbar^T, Poisson-chain scratch
     bool adj;
+    // cluster-resident step (vv_cluster.cuh): the shape of a single run (ctas 0:
+    // the multi-kernel path), slot-ordered LU tables, the instance description
+    // on the device and its host copy, squared LU multipliers per v row
+    // (largest over the modes: carry levels of any shape)
+    vv::ClShape cls;
+    void *cl_dinv, *cl_lam;
+    double* cl_green;
+    vv::ClInst *cl_dev, *cl_host;
+    bool cl_sent;
+    std::vector<double> *cl_lf, *cl_lb;
     double *adj_cH, *adj_cF, *adj_zpart, *adj_zbuf, *adj_q, *adj_hprof, *adj_h1a, *adj_h1b;
 };
 
@@ -1607,6 +1619,120 @@ int step_host(vv_ctx* c, vv_state* st) {
     return VV_OK;
 }
 
+// ---- cluster-resident step ------------------------------------------------------
+// CTAs of a single run's cluster (VV_CLUSTER=n fixes it; 0: the multi-kernel
+// path, which the tests compare with).  Sixteen wherever the instance fits:
+// two steps of 64 x 256 in FP64 take 498 us on 16 CTAs, 524 on 8, 622 on 4
+// and 1417 in the multi-kernel graph; 256 x 512, the largest that fits in
+// FP64, 1670 against 2240.  The direct-DFT rows cost rows nx^2 per CTA and
+// lose from about a million on (300 x 100, 0.63 M: 1.9x faster; 200 x 400,
+// 1.0 M: even; 201 x 401, 1.05 M: 7% slower).
+int cl_default_ctas(const vv_ctx* c) {
+    const int rows = (c->nv + vv::CL_MAXC - 1) / vv::CL_MAXC;
+    const bool dft = !(c->pow2 && c->nx >= 64);
+    return dft && (double)rows * c->nx * c->nx > 9e5 ? 0 : vv::CL_MAXC;
+}
+
+// configurations the cluster kernel covers: the factored Arakawa brackets with
+// the point time derivative and the kinetic preconditioner
+bool cl_covers(const vv_ctx* c) {
+    return c->g.preconditioner == VV_PC_TENSOR_KINETIC && c->g.order != VV_ORDER_REFERENCE &&
+           c->g.bracket != VV_BRACKET_SIMPSON && c->avg == vv::AVG_POINT && c->coll == vv::COLL_NONE && !c->db &&
+           !c->pred && c->restart <= vv::CL_RESTART && c->nx <= vv::CL_NXMAX;
+}
+
+double cl_tol(const vv_ctx* c) { return c->mixed ? 1e-10 : 1e-18; }
+
+// the description of context c as one instance of shape sh
+void cl_describe(const vv_ctx* c, const vv::ClShape& sh, const vv_state* st, vv::ClInst* I) {
+    std::memset((void*)I, 0, sizeof *I);
+    I->ds = c->ds;
+    I->nx = c->nx;
+    I->nv = c->nv;
+    I->fam = sh.fam;
+    I->rows = sh.rows;
+    I->nch = sh.nch;
+    I->kv = sh.kv;
+    I->dsm = sh.dsm;
+    I->klev = vv::cl_levels(sh, c->nv, c->cl_lf->data(), c->cl_lb->data(), cl_tol(c));
+    I->restart = c->restart;
+    I->ncell = c->ncell;
+    I->ht_inv = c->ht_inv;
+    I->hv = c->hv;
+    switch (c->g.bracket) {
+        case VV_BRACKET_J1: I->scheme = 1; I->fscale = c->f1; I->cA1 = vv::Coef<1>::cA1; I->cA2 = vv::Coef<1>::cA2; break;
+        case VV_BRACKET_J2: I->scheme = 2; I->fscale = c->f2; I->cA1 = vv::Coef<2>::cA1; I->cA2 = vv::Coef<2>::cA2; break;
+        default: I->scheme = 4; I->fscale = c->f1; I->cA1 = vv::Coef<4>::cA1; I->cA2 = vv::Coef<4>::cA2; break;
+    }
+    I->h0 = c->h0;
+    I->v = c->v;
+    I->hxp = c->hxp;
+    I->tw = c->mixed ? (const void*)c->tw32 : (const void*)c->tw;
+    I->dinv = c->cl_dinv;
+    I->lam = c->cl_lam;
+    I->alpha = c->mixed ? (const void*)c->alpha32 : (const void*)c->alpha;
+    I->gamma = c->mixed ? (const void*)c->gamma32 : (const void*)c->gamma;
+    I->green = c->cl_green;
+    I->po = pparams(c);
+    I->Fh = c->Fh;
+    I->fl = c->fl;
+    if (c->mixed) {
+        I->V = c->V32; I->bT = c->bvec32; I->xT = c->delta32;
+    } else {
+        I->V = c->V; I->bT = c->bvec; I->xT = c->delta;
+    }
+    if (st) {
+        I->f = st->f; I->fh = st->fh; I->phi = st->phi; I->phih = st->phih;
+        I->h1c = st->h1c; I->h1h = st->h1h; I->h2c = st->h2c; I->h2h = st->h2h;
+        I->n = st->n; I->u = st->u; I->e = st->e; I->a = st->a;
+    }
+}
+
+// slot-ordered tables of a context (vv_create, and a batch of contexts
+// created for the multi-kernel path)
+int cl_prepare(vv_ctx* c, const vv::ClShape& sh) {
+    if (c->cl_dinv) return VV_OK;
+    const size_t csz = c->mixed ? sizeof(float2) : sizeof(double2);
+    // one allocation: tables, the instance's description
+    auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
+    const size_t nd = al((size_t)c->nv * sh.slots * csz), nl = al((size_t)sh.slots * csz);
+    char* base = nullptr;
+    TRY(dalloc(&base, nd + nl + sizeof(vv::ClInst)));
+    c->cl_dinv = base;
+    c->cl_lam = base + nd;
+    c->cl_dev = reinterpret_cast<vv::ClInst*>(base + nd + nl);
+    if (!c->cl_host) c->cl_host = new vv::ClInst();
+    const cudaError_t e = vv::cl_tables(c->mixed, sh, c->nv, c->mixed ? (const void*)c->dinv32 : (const void*)c->dinv,
+                                        c->mixed ? (const void*)c->lambda32 : (const void*)c->lambda, c->cl_dinv,
+                                        c->cl_lam, c->g.ht, 0);
+    return e == cudaSuccess ? VV_OK : fail_cuda(e, "cluster tables");
+}
+
+// run the context's instance: the step of st, or the solve of b -> x
+int cl_run_single(vv_ctx* c, const vv_state* st, const void* b, void* x) {
+    vv::ClInst I;
+    I = *c->cl_host;
+    if (st) {
+        I.f = st->f; I.fh = st->fh; I.phi = st->phi; I.phih = st->phih;
+        I.h1c = st->h1c; I.h1h = st->h1h; I.h2c = st->h2c; I.h2h = st->h2h;
+        I.n = st->n; I.u = st->u; I.e = st->e; I.a = st->a;
+        I.bT = c->mixed ? (void*)c->bvec32 : (void*)c->bvec;
+        I.xT = c->mixed ? (void*)c->delta32 : (void*)c->delta;
+    } else {
+        I.bT = const_cast<void*>(b);
+        I.xT = x;
+    }
+    if (std::memcmp((const void*)&I, (const void*)c->cl_host, sizeof I) != 0 || !c->cl_sent) {
+        std::memcpy((void*)c->cl_host, (const void*)&I, sizeof I);
+        CK(cudaMemcpyAsync(c->cl_dev, c->cl_host, sizeof I, cudaMemcpyHostToDevice, c->st));
+        c->cl_sent = true;
+    }
+    const cudaError_t e = vv::cl_launch(c->mixed, c->cls.fam, c->cl_dev, nullptr, 1, c->cls.ctas, c->cls.smem,
+                                        st ? vv::CL_STEP : vv::CL_GMRES, c->st);
+    c->launches++;
+    return e == cudaSuccess ? VV_OK : fail_cuda(e, "cluster launch");
+}
+
 }  // namespace
 
 // =============================================================================
@@ -1760,7 +1886,7 @@ int vv_create(const vv_grid* grid, vv_ctx** out) {
         (s = dalloc(&c->mom_part, (size_t)c->mom_S * 3 * nx)) || (s = dalloc(&c->spec, (size_t)nm * nv)) ||
         (s = dalloc(&c->tw, (size_t)nx)) || (s = dalloc(&c->lambda, nm)) ||
         (s = dalloc(&c->dinv, (size_t)nm * nv)) || (s = dalloc(&c->alpha, nv)) || (s = dalloc(&c->gamma, nv)) ||
-        (s = dalloc(&c->sym_inv, nm)) || (s = dalloc(&c->ds, 1))) {
+        (s = dalloc(&c->sym_inv, (size_t)nm + nx)) || (s = dalloc(&c->ds, 1))) {
         vv_destroy(c);
         return s;
     }
@@ -1809,6 +1935,7 @@ int vv_create(const vv_grid* grid, vv_ctx** out) {
     }
     std::vector<double2> dinv((size_t)nm * nv);
     std::vector<double2> lam2(nm);
+    const bool covers = cl_covers(c);
     bool piv = false;
     for (int k = 0; k < nm; ++k) {
         const cd L = lam[k];
@@ -1987,6 +2114,51 @@ int vv_create(const vv_grid* grid, vv_ctx** out) {
         const char* e = getenv("VV_MARCH");   // fixed strip width (tests, profiling); the autotuner may override
         if (e) c->march = atoi(e);
     }
+    if (covers) {
+        // |l_j| = |lambda alpha_j / U_{j-1}|, |m_j| = |lambda gamma_j / U_j|
+        std::vector<double> mult(nv, 0.0);   // max over the modes of |lambda / U_j|^2
+        for (int k = 0; k < nm; ++k) {
+            const double l2 = lam2[k].x * lam2[k].x + lam2[k].y * lam2[k].y;
+            const double2* d = dinv.data() + (size_t)k * nv;
+            for (int j = 0; j < nv; ++j) mult[j] = std::max(mult[j], l2 * (d[j].x * d[j].x + d[j].y * d[j].y));
+        }
+        c->cl_lf = new std::vector<double>(nv, 0.0);
+        c->cl_lb = new std::vector<double>(nv, 0.0);
+        for (int j = 0; j < nv; ++j) {
+            if (j > 0) (*c->cl_lf)[j] = alpha[j] * alpha[j] * mult[j - 1];
+            if (j + 1 < nv) (*c->cl_lb)[j] = gamma[j] * gamma[j] * mult[j];
+        }
+        // the circulant inverse of the Laplacian on mean-free profiles, symmetric:
+        // green_d = (1/nx) sum_k cos(2 pi k d / nx) / symbol_k
+        std::vector<double> green(nx), inv(nx / 2 + 1);
+        for (int k = 1; 2 * k <= nx; ++k)
+            inv[k] = 1.0 / ((c->lap[0] + 2. * c->lap[1] * tw[k].x + 2. * c->lap[2] * tw[2 * k % nx].x) * c->hx2_inv /
+                            c->lap[3]);
+        for (int d = 0; d <= nx / 2; ++d) {
+            double t = 0.0;
+            for (int k = 1; 2 * k <= nx; ++k) t += (2 * k == nx ? 1.0 : 2.0) * inv[k] * tw[(size_t)k * d % nx].x;
+            green[d] = green[(nx - d) % nx] = t / nx;
+        }
+        c->cl_green = c->sym_inv + nm;
+        if (cudaMemcpy(c->cl_green, green.data(), nx * sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess) {
+            vv_destroy(c);
+            return fail_cuda(cudaGetLastError(), "vv_create upload");
+        }
+        const char* sh = getenv("VV_SHAPE");
+        const char* ec = getenv("VV_CLUSTER");
+        const int ctas = ec && ec[0] ? atoi(ec) : cl_default_ctas(c);
+        if (!(sh && sh[0]) && ctas > 0) {
+            const vv::ClShape t = vv::cl_shape(nx, nv, c->pow2, ctas, c->mixed ? 4 : 8, vv::cl_smem_limit(c->mixed));
+            if (t.ctas && vv::cl_resident(c->mixed, t.fam, t.ctas, t.smem) > 0) {
+                if ((s = cl_prepare(c, t)) != VV_OK) {
+                    vv_destroy(c);
+                    return s;
+                }
+                c->cls = t;
+                cl_describe(c, t, nullptr, c->cl_host);
+            }
+        }
+    }
     {
         // VV_SHAPE="fft,R,tri,narrow[,march]" fixes the kernel variants (tests run each variant
         // explicitly; profiling); else the autotuner picks them by timing
@@ -2022,7 +2194,10 @@ int vv_destroy(vv_ctx* c) {
                     c->adj_zbuf, c->adj_q, c->adj_hprof, c->adj_h1a, c->adj_h1b, c->lamv, c->twv, c->pv_spec,
                     c->pv_scr, c->pv_xt, c->phipc, c->twv32, c->pv_spec32, c->pv_scr32, c->pv_xt32,
                     c->mom_p, c->mom_h, c->db_fave, c->db_b, c->pred_H, c->pred_Hp, c->pred_Y, c->pred_K,
-                    c->pred_S, c->pred_fl, c->pred_cpart, c->pred_zero};
+                    c->pred_S, c->pred_fl, c->pred_cpart, c->pred_zero, c->cl_dinv};
+    delete c->cl_host;
+    delete c->cl_lf;
+    delete c->cl_lb;
     destroy_graph(c);
     for (int k = 0; k < 4; ++k)
         if (c->cs[k]) cudaStreamDestroy(c->cs[k]);
@@ -2179,6 +2354,24 @@ int vv_gmres(vv_ctx* c, const double* b, double* x, const vv_ksp_opts* o, vv_ksp
     c->opts_valid = false;
     for (int k = 0; k < 5; ++k) c->hnd[k] = saved[k];
     TRY(s);
+    if (c->cls.ctas && restart <= vv::CL_RESTART && (c->mixed || (aligned16(b) && aligned16(x) && b != x))) {
+        if (c->mixed) {
+            vv::k_scale<double, float><<<grid1d(c->ncell, 256), 256, 0, c->st>>>(b, c->bvec32, c->ncell, nullptr, 1.0);
+            CKL(c);
+            TRY(cl_run_single(c, nullptr, c->bvec32, c->delta32));
+            vv::k_scale<float, double><<<grid1d(c->ncell, 256), 256, 0, c->st>>>(c->delta32, x, c->ncell, nullptr, 1.0);
+            CKL(c);
+        } else {
+            TRY(cl_run_single(c, nullptr, b, x));
+        }
+        GmHead h{};
+        CK(cudaMemcpyAsync(c->hpin, &c->ds->res, sizeof(double), cudaMemcpyDeviceToHost, c->st));
+        TRY(read_head(c, &h));
+        r->its = h.its;
+        r->reason = h.reason;
+        r->rnorm = c->hpin[0];
+        return VV_OK;
+    }
     if (!c->mixed) return gmres_host<double>(c, b, x, r);
     // mixed: FP32 solve of the FP64 system, converted at the boundary
     vv::k_scale<double, float><<<grid1d(c->ncell, 256), 256, 0, c->st>>>(b, c->bvec32, c->ncell, nullptr, 1.0);
@@ -2314,7 +2507,12 @@ int vv_step(vv_ctx* c, vv_state* st, const vv_snes_opts* so, const vv_ksp_opts* 
         c->coll_p = {st->n, st->u, st->a};
     }
     std::memset(rep, 0, sizeof(*rep));
-    if (c->use_graph) {
+    const bool cluster = c->cls.ctas && restart <= vv::CL_RESTART;
+    if (cluster) {
+        for (auto& h : c->hnd) h = 0;
+        TRY(upload_options(c, ko, so));
+        TRY(cl_run_single(c, st, nullptr, nullptr));
+    } else if (c->use_graph) {
         if (!c->step_exec || !same_state(c->step_key, *st)) TRY(build_step_graph(c, st));
         std::memcpy(c->hnd, c->step_hnd, sizeof c->hnd);
         TRY(upload_options(c, ko, so));
@@ -2330,7 +2528,7 @@ int vv_step(vv_ctx* c, vv_state* st, const vv_snes_opts* so, const vv_ksp_opts* 
     // report
     CK(cudaMemcpyAsync(c->hds, c->ds, offsetof(vv::DevState, hcol), cudaMemcpyDeviceToHost, c->st));
     CK(cudaStreamSynchronize(c->st));
-    return fill_report(c, *c->hds, restart, rep, so->abort_residual);
+    return fill_report(c, *c->hds, restart, rep, so->abort_residual, !cluster);
 }
 
 int vv_invariants(vv_ctx* c, const double* f, const double* phi, const double* h2, vv_invariant_set* out) {
@@ -2509,6 +2707,29 @@ struct vv_batch {
     cudaGraphExec_t ex;
     unsigned long long hnd[4];   // batch handles: pic, outer, inner, revert (index = BH_*)
     bool use_graph;
+    // cluster-resident batch (vv_cluster.cuh): every instance that fits steps on
+    // its own cluster, one launch per class of (row kind, CTAs); the others as
+    // the lockstep batch `rest`.  `lock`: a lockstep batch of the whole table,
+    // made when a lockstep kernel is to be timed.
+    bool cl;
+    struct ClClass {
+        int fam, ctas;
+        size_t smem;
+        std::vector<int> inst;   // longest first
+        int* order;              // device: indices into cltab
+        cudaStream_t st;
+        cudaEvent_t done;
+    };
+    std::vector<ClClass> classes;
+    vv::ClInst* cltab;
+    int* horder;                 // pinned staging of the classes' orders
+    cudaEvent_t fork, rest_done;
+    cudaStream_t rest_st;
+    std::vector<double> cost;    // per instance: the last step's work (cells x GMRES iterations)
+    std::vector<int> rest_idx;
+    std::vector<vv_step_report> rest_rep;
+    std::vector<int> rest_status;
+    vv_batch *rest, *lock;
     int64_t launches;
     int64_t pending_l0 = 0;      // launch count before the uncollected launch
     int pending = 0;             // 1: a vv_batch_launch awaits its vv_batch_collect
@@ -3043,6 +3264,19 @@ extern "C" {
 int vv_batch_destroy(vv_batch* b) {
     if (!b) return VV_OK;
     if (b->pending && b->user) cudaStreamSynchronize(b->user);   // a launch never collected: let it finish
+    vv_batch_destroy(b->rest);
+    vv_batch_destroy(b->lock);
+    for (auto& c : b->classes) {
+        if (c.st) cudaStreamSynchronize(c.st);
+        if (c.done) cudaEventDestroy(c.done);
+        if (c.st) cudaStreamDestroy(c.st);
+        if (c.order) cudaFree(c.order);
+    }
+    if (b->fork) cudaEventDestroy(b->fork);
+    if (b->rest_done) cudaEventDestroy(b->rest_done);
+    if (b->rest_st) cudaStreamDestroy(b->rest_st);
+    if (b->cltab) cudaFree(b->cltab);
+    if (b->horder) cudaFreeHost(b->horder);
     for (auto s : b->cs) {
         cudaStreamCaptureStatus cst = cudaStreamCaptureStatusNone;
         if (s && cudaStreamIsCapturing(s, &cst) == cudaSuccess && cst != cudaStreamCaptureStatusNone) {
@@ -3065,9 +3299,14 @@ int vv_batch_destroy(vv_batch* b) {
     return VV_OK;
 }
 
-int vv_batch_create(int n, vv_ctx* const* ctxs, const vv_state* states, vv_batch** out) {
-    if (n < 1 || !ctxs || !states || !out) return VV_ERR_ARG;
-    *out = nullptr;
+}  // extern "C"
+
+namespace {
+
+int lockstep_create(int n, vv_ctx* const* ctxs, const vv_state* states, vv_batch** out);
+
+// what a batch accepts
+int batch_check(int n, vv_ctx* const* ctxs, const vv_state* states) {
     for (int i = 0; i < n; ++i) {
         const vv_state& s = states[i];
         if (!ctxs[i] || !s.f || !s.fh || !s.phi || !s.h1c || !s.h1h || !s.n) return VV_ERR_ARG;
@@ -3086,6 +3325,151 @@ int vv_batch_create(int n, vv_ctx* const* ctxs, const vv_state* states, vv_batch
             c->pred || c->nx % vv::WX != 0 || !c->pow2 || c->device != c0->device)
             return VV_ERR_UNSUPPORTED;
     }
+    return VV_OK;
+}
+
+// CTAs of an instance's cluster in a batch.  There the sum of the work counts
+// and not one instance's latency: wide clusters spend more of their time at
+// barriers, so an instance gets the fewest CTAs that hold it at a reasonable
+// step time.  256-instance sweep, mixed, three steps from the start / later
+// steps: 115 / 27 ms with 16 CTAs each, 104 / 23 with 16 from 64 K cells and 8
+// from 16 K, 92 / 18.6 with these lines.
+int cl_batch_ctas(const vv_ctx* c) {
+    return c->ncell >= 200000 ? 16 : c->ncell >= 65536 ? 8 : c->ncell >= 16384 ? 4 : 2;
+}
+
+// classes, tables and streams of a cluster-resident batch; the instances that
+// fit no cluster go to rest_idx
+int cl_batch_build(vv_batch* b) {
+    const int n = b->n;
+    std::vector<vv::ClInst> tab(n);
+    b->cost.assign(n, 0.0);
+    for (int i = 0; i < n; ++i) {
+        vv_ctx* c = b->ctx[i];
+        vv::ClShape t{};
+        if (c->cl_lf)
+            for (int ctas = cl_batch_ctas(c); ctas <= vv::CL_MAXC && !t.ctas; ctas *= 2) {
+                t = vv::cl_shape(c->nx, c->nv, c->pow2, ctas, c->mixed ? 4 : 8, vv::cl_smem_limit(c->mixed));
+                if (t.ctas && vv::cl_resident(c->mixed, t.fam, t.ctas, t.smem) < 1) t = vv::ClShape{};
+            }
+        b->cost[i] = (double)c->ncell;
+        if (!t.ctas) {
+            b->rest_idx.push_back(i);
+            continue;
+        }
+        TRY(cl_prepare(c, t));
+        cl_describe(c, t, &b->states[i], &tab[i]);
+        vv_batch::ClClass* k = nullptr;
+        for (auto& q : b->classes)
+            if (q.fam == t.fam && q.ctas == t.ctas) k = &q;
+        if (!k) {
+            b->classes.push_back({t.fam, t.ctas, 0, {}, nullptr, nullptr, nullptr});
+            k = &b->classes.back();
+        }
+        k->smem = std::max(k->smem, t.smem);
+        k->inst.push_back(i);
+    }
+    if (b->classes.empty()) return VV_OK;
+    // the widest clusters are placed first
+    std::sort(b->classes.begin(), b->classes.end(), [](const vv_batch::ClClass& x, const vv_batch::ClClass& y) {
+        return x.ctas != y.ctas ? x.ctas > y.ctas : x.fam > y.fam;
+    });
+    int lo = 0, hi = 0;
+    CK(cudaDeviceGetStreamPriorityRange(&lo, &hi));
+    CK(cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming));
+    CK(cudaMallocHost((void**)&b->horder, n * sizeof(int)));
+    int s = upload_vec(&b->cltab, tab);
+    if (s != VV_OK) return s;
+    for (auto& k : b->classes) {
+        CK(cudaStreamCreateWithPriority(&k.st, cudaStreamNonBlocking, k.ctas == vv::CL_MAXC ? hi : lo));
+        CK(cudaEventCreateWithFlags(&k.done, cudaEventDisableTiming));
+        if ((s = dalloc(&k.order, k.inst.size())) != VV_OK) return s;
+    }
+    return VV_OK;
+}
+
+// launch every class on its stream, forked from and joined to the user's
+int cl_batch_launch(vv_batch* b) {
+    CK(cudaEventRecord(b->fork, b->user));
+    int off = 0;
+    for (auto& k : b->classes) {
+        std::stable_sort(k.inst.begin(), k.inst.end(), [&](int x, int y) { return b->cost[x] > b->cost[y]; });
+        for (size_t q = 0; q < k.inst.size(); ++q) b->horder[off + q] = k.inst[q];
+        CK(cudaStreamWaitEvent(k.st, b->fork, 0));
+        CK(cudaMemcpyAsync(k.order, b->horder + off, k.inst.size() * sizeof(int), cudaMemcpyHostToDevice, k.st));
+        const cudaError_t e = vv::cl_launch(b->mixed, k.fam, b->cltab, k.order, (int)k.inst.size(), k.ctas, k.smem,
+                                            vv::CL_STEP, k.st);
+        if (e != cudaSuccess) return fail_cuda(e, "cluster launch");
+        b->launches++;
+        CK(cudaEventRecord(k.done, k.st));
+        off += (int)k.inst.size();
+    }
+    for (auto& k : b->classes) CK(cudaStreamWaitEvent(b->user, k.done, 0));
+    return VV_OK;
+}
+
+}  // namespace
+
+extern "C" {
+
+int vv_batch_create(int n, vv_ctx* const* ctxs, const vv_state* states, vv_batch** out) {
+    if (n < 1 || !ctxs || !states || !out) return VV_ERR_ARG;
+    const char* bs = getenv("VV_BATCH_SHAPE");
+    const char* ec = getenv("VV_CLUSTER");
+    // the checks of the lockstep batch hold for both kinds
+    const int ok = batch_check(n, ctxs, states);
+    if (ok != VV_OK || (bs && bs[0]) || (ec && ec[0] == '0')) return lockstep_create(n, ctxs, states, out);
+    *out = nullptr;
+    vv_batch* b = new vv_batch();
+    b->n = n;
+    b->ctx.assign(ctxs, ctxs + n);
+    b->states.assign(states, states + n);
+    b->mixed = ctxs[0]->mixed;
+    b->cl = true;
+    auto fail_b = [&](int code) { vv_batch_destroy(b); return code; };
+    int r = cl_batch_build(b);
+    if (r != VV_OK) return fail_b(r);
+    if (b->classes.empty()) {   // nothing fits
+        vv_batch_destroy(b);
+        return lockstep_create(n, ctxs, states, out);
+    }
+    if (!b->rest_idx.empty()) {
+        std::vector<vv_ctx*> rc;
+        std::vector<vv_state> rs;
+        for (int i : b->rest_idx) {
+            rc.push_back(ctxs[i]);
+            rs.push_back(states[i]);
+        }
+        if (cudaStreamCreateWithFlags(&b->rest_st, cudaStreamNonBlocking) != cudaSuccess ||
+            cudaEventCreateWithFlags(&b->rest_done, cudaEventDisableTiming) != cudaSuccess)
+            return fail_b(fail_cuda(cudaGetLastError(), "batch stream"));
+        b->rest_rep.resize(rc.size());
+        b->rest_status.resize(rc.size());
+        if ((r = lockstep_create((int)rc.size(), rc.data(), rs.data(), &b->rest)) != VV_OK) return fail_b(r);
+    }
+    std::vector<vv::BInst> tab(n);
+    for (int i = 0; i < n; ++i) {
+        std::memset(&tab[i], 0, sizeof tab[i]);
+        tab[i].ds = ctxs[i]->ds;
+    }
+    if ((r = upload_vec(&b->tab, tab))) return fail_b(r);
+    b->words = (int)(offsetof(vv::DevState, hcol) / sizeof(unsigned int));
+    if (cudaMalloc((void**)&b->gather, (size_t)n * b->words * sizeof(unsigned int)) != cudaSuccess ||
+        cudaMallocHost((void**)&b->hgather, (size_t)n * b->words * sizeof(unsigned int)) != cudaSuccess)
+        return fail_b(VV_ERR_ALLOC);
+    *out = b;
+    return VV_OK;
+}
+
+}  // extern "C"
+
+namespace {
+
+int lockstep_create(int n, vv_ctx* const* ctxs, const vv_state* states, vv_batch** out) {
+    if (n < 1 || !ctxs || !states || !out) return VV_ERR_ARG;
+    *out = nullptr;
+    TRY(batch_check(n, ctxs, states));
+    const vv_ctx* c0 = ctxs[0];
     vv_batch* b = new vv_batch();   // value-initialised: pointers and counts start at zero
     b->n = n;
     b->ctx.assign(ctxs, ctxs + n);
@@ -3293,6 +3677,10 @@ int vv_batch_create(int n, vv_ctx* const* ctxs, const vv_state* states, vv_batch
     return VV_OK;
 }
 
+}  // namespace
+
+extern "C" {
+
 int vv_batch_set_stream(vv_batch* b, void* stream) {
     if (!b) return VV_ERR_ARG;
     b->user = (cudaStream_t)stream;
@@ -3316,6 +3704,23 @@ int vv_batch_launch(vv_batch* b, const vv_snes_opts* so, const vv_ksp_opts* ko) 
     }
     b->st = b->user;
     b->pending_l0 = b->launches;
+    if (b->cl) {
+        TRY(cl_batch_launch(b));
+        if (b->rest) {   // beside the clusters
+            b->rest->user = b->rest_st;
+            CK(cudaStreamWaitEvent(b->rest_st, b->fork, 0));
+            TRY(vv_batch_launch(b->rest, so, ko));
+            CK(cudaEventRecord(b->rest_done, b->rest_st));
+            CK(cudaStreamWaitEvent(b->user, b->rest_done, 0));
+        }
+        vv::k_b_gather_states<<<b->n, 128, 0, b->user>>>(b->tab, b->words, b->gather);
+        b->launches++;
+        CK(cudaGetLastError());
+        CK(cudaMemcpyAsync(b->hgather, b->gather, (size_t)b->n * b->words * sizeof(unsigned int),
+                           cudaMemcpyDeviceToHost, b->user));
+        b->pending = 1;
+        return VV_OK;
+    }
     CK(cudaMemsetAsync(b->counts, 0, vv::BN_WORDS * sizeof(unsigned int), b->user));
     if (b->use_graph) {
         CK(cudaGraphLaunch(b->ex, b->user));
@@ -3341,6 +3746,12 @@ int vv_batch_collect(vv_batch* b, const vv_snes_opts* so, const vv_ksp_opts* ko,
     if (!b || !so || !ko || !reports) return VV_ERR_ARG;
     if (!b->pending) return fail(VV_ERR_ARG, "vv_batch_collect: nothing launched");
     b->pending = 0;
+    if (b->rest) {
+        const int r = vv_batch_collect(b->rest, so, ko, b->rest_rep.data(), b->rest_status.data());
+        if (r != VV_OK && r != VV_ERR_DIVERGED && r != VV_ERR_NAN) return r;
+        b->launches += b->rest->launches;
+        b->rest->launches = 0;
+    }
     CK(cudaStreamSynchronize(b->user));
     if (b->use_graph) {
         const unsigned* k = b->hcounts;
@@ -3356,7 +3767,15 @@ int vv_batch_collect(vv_batch* b, const vv_snes_opts* so, const vv_ksp_opts* ko,
         vv_ctx* c = b->ctx[i];
         std::memcpy(&d, b->hgather + (size_t)i * b->words, (size_t)b->words * sizeof(unsigned int));
         const int restart = (ko->restart > 0) ? ko->restart : c->restart;
-        const int s = fill_report(c, d, restart, &reports[i], so->abort_residual, false);
+        int s = fill_report(c, d, restart, &reports[i], so->abort_residual, false);
+        if (b->cl) {
+            b->cost[i] = (double)c->ncell * (reports[i].gmres_its_total + reports[i].picard_its);
+            for (size_t q = 0; q < b->rest_idx.size(); ++q)
+                if (b->rest_idx[q] == i) {
+                    reports[i] = b->rest_rep[q];
+                    s = b->rest_status[q];
+                }
+        }
         if (statuses) statuses[i] = s;
         if (s != VV_OK && first_bad == VV_OK) first_bad = s;
     }
@@ -3374,6 +3793,10 @@ int vv_batch_time_kernel(vv_batch* b, int which, int it, int reps, double* avg_m
     if (!b || !avg_ms || reps < 1 || which < 0 || which > 5 || it < 0) return VV_ERR_ARG;
     for (int i = 0; i < b->n; ++i)
         if (it + 1 >= b->ctx[i]->restart + 1) return VV_ERR_ARG;   // V[it+1] must exist
+    if (b->cl) {   // the lockstep kernels of the same table
+        if (!b->lock) TRY(lockstep_create(b->n, b->ctx.data(), b->states.data(), &b->lock));
+        return vv_batch_time_kernel(b->lock, which, it, reps, avg_ms);
+    }
     const int64_t l0 = b->launches;
     b->st = b->cs[0];
     vv::k_b_set_it<<<1, 256, 0, b->st>>>(b->tab, b->n, it);

@@ -125,7 +125,7 @@ k_sum_partial(const T* __restrict__ x, size_t n, double* __restrict__ part) {
 }
 
 // Reduce `np` partials per column (m columns, stride ld) into out[m].
-__global__ void __launch_bounds__(RED_THREADS)
+static __global__ void __launch_bounds__(RED_THREADS)
 k_reduce_cols(const double* __restrict__ part, int np, int m, int ld, double* __restrict__ out) {
     const int w = threadIdx.x >> 5;
     for (int q = w; q < m; q += RED_THREADS / 32) {
@@ -502,7 +502,7 @@ __device__ __forceinline__ void pic_residual_warp(DevState* s, const double* __r
     set_cond(s->h_pic, s->pic_active ? 1u : 0u);
     set_cond(s->h_revert, (unsigned)s->pic_revert);
 }
-__global__ void k_pic_residual(DevState* s, const double* __restrict__ part, int np, int phase) {
+static __global__ void k_pic_residual(DevState* s, const double* __restrict__ part, int np, int phase) {
     pic_residual_warp(s, part, np, phase);
 }
 
@@ -576,12 +576,13 @@ constexpr int POIS_THREADS = 1024;
 // Single CTA.  Inputs: moment partials (or n directly when part == nullptr).
 // Outputs (each optional): n, u, e, a, phi, h1; scal[0] = ||Poisson residual||_2,
 // scal[1] = sum(phi).
-__device__ __forceinline__ void moments_poisson_cta(const double* __restrict__ part, const double* __restrict__ n_in,
-                                                    double* __restrict__ n, double* __restrict__ u,
-                                                    double* __restrict__ e, double* __restrict__ a,
-                                                    double* __restrict__ phi, double* __restrict__ h1,
-                                                    double* __restrict__ scal, const PoissonParams& p) {
-    extern __shared__ double2 psm[];
+// psm: the scratch, M + 1 complex, nx (padded to even) and nx + 2 doubles.
+__device__ __forceinline__ void moments_poisson_core(double2* psm, const double* __restrict__ part,
+                                                     const double* __restrict__ n_in, double* __restrict__ n,
+                                                     double* __restrict__ u, double* __restrict__ e,
+                                                     double* __restrict__ a, double* __restrict__ phi,
+                                                     double* __restrict__ h1, double* __restrict__ scal,
+                                                     const PoissonParams& p) {
     double2* buf = psm;                                   // M + 1 complex
     double* nn = reinterpret_cast<double*>(psm + p.M + 1);  // nx, padded to an even count
     double* ph = nn + ((p.nx + 1) & ~1);                  // nx + 2; 16-byte aligned (read as double2)
@@ -723,7 +724,15 @@ __device__ __forceinline__ void moments_poisson_cta(const double* __restrict__ p
         scal[1] = phisum_s;
     }
 }
-__global__ void __launch_bounds__(POIS_THREADS)
+__device__ __forceinline__ void moments_poisson_cta(const double* __restrict__ part, const double* __restrict__ n_in,
+                                                    double* __restrict__ n, double* __restrict__ u,
+                                                    double* __restrict__ e, double* __restrict__ a,
+                                                    double* __restrict__ phi, double* __restrict__ h1,
+                                                    double* __restrict__ scal, const PoissonParams& p) {
+    extern __shared__ double2 psm[];
+    moments_poisson_core(psm, part, n_in, n, u, e, a, phi, h1, scal, p);
+}
+static __global__ void __launch_bounds__(POIS_THREADS)
 k_moments_poisson(const double* __restrict__ part, const double* __restrict__ n_in,
                   double* __restrict__ n, double* __restrict__ u, double* __restrict__ e,
                   double* __restrict__ a, double* __restrict__ phi, double* __restrict__ h1,
@@ -777,7 +786,7 @@ constexpr int INV_SUMS = 13;   // mass, L1..L6, L8, S, Ekin, Ep1, Ep2, P
 constexpr int INV_NPART = INV_SUMS + 2;  // + min, max
 
 // one CTA: h1 = phi - mean(phi) into h1out, field energy into fe[0]
-__global__ void k_xprofile(const double* __restrict__ phi, int nx, double charge, double hx,
+static __global__ void k_xprofile(const double* __restrict__ phi, int nx, double charge, double hx,
                            double* __restrict__ h1out, double* __restrict__ fe) {
     __shared__ double red[32];
     __shared__ double mean_s;
@@ -796,7 +805,7 @@ __global__ void k_xprofile(const double* __restrict__ phi, int nx, double charge
     if (threadIdx.x == 0) fe[0] = 0.5 * charge * w / hx;
 }
 
-__global__ void __launch_bounds__(RED_THREADS)
+static __global__ void __launch_bounds__(RED_THREADS)
 k_invariants_partial(const double* __restrict__ f, int nx, int nv, const double* __restrict__ v,
                      const double* __restrict__ h0, const double* __restrict__ h1,
                      const double* __restrict__ h2, double* __restrict__ part) {
@@ -852,7 +861,7 @@ k_invariants_partial(const double* __restrict__ f, int nx, int nv, const double*
 }
 
 // one CTA: out[q] for the 13 sums (compensated over partials), min, max
-__global__ void __launch_bounds__(RED_THREADS)
+static __global__ void __launch_bounds__(RED_THREADS)
 k_invariants_final(const double* __restrict__ part, int np, double* __restrict__ out) {
     __shared__ double sh[RED_THREADS / 32];
     for (int q = 0; q < INV_SUMS; ++q) {
