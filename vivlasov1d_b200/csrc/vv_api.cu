@@ -15,6 +15,7 @@
 #include "vv_batch.cuh"
 #include "vv_adjoint.cuh"
 #include "vv_pcv.cuh"
+#include "vv_pcl.cuh"
 #include "vv_coll.cuh"
 #include "vv_pred.cuh"
 #include "vv_cluster.h"
@@ -92,6 +93,11 @@ struct vv_ctx {
     bool pow2;         // nx a power of two
     int tri_kind;      // 0: one CTA per mode (block scan), 1: one warp per mode (lines staged in shared
                        // memory when tri_ws_smem fits smem_limit)
+    // v-major preconditioner (vv_pcl.cuh), in the GMRES precision: 1 when in use;
+    // its LU table, second spectrum and carry levels (chunks of 16 and of 8 rows)
+    int vmaj;
+    void *vm_dinv, *vm_spec;
+    int vm_lev16, vm_lev8;
     int smem_limit;    // dynamic shared memory per block on this device
     int narrow_bracket;  // 1: 32x16 tiles instead of 64x32
     int march;           // Jacobian stencil: 0 tiles, 128 or 256 the strip width of the marching kernel
@@ -620,6 +626,27 @@ int raise_smem_limits(int* limit_out) {
         smem_attributes<double>(optin, lowest, e);
         smem_attributes<float>(optin, lowest, e);
         smem_set((const void*)vv::k_moments_poisson, optin, lowest, e);
+#define VV_SETL(M)                                                          \
+    smem_set((const void*)vv::k_rfftl<double, double, M>, optin, lowest, e);  \
+    smem_set((const void*)vv::k_rfftl<double, float, M>, optin, lowest, e);   \
+    smem_set((const void*)vv::k_rfftl<float, float, M>, optin, lowest, e);    \
+    smem_set((const void*)vv::k_irfftl<double, double, M>, optin, lowest, e); \
+    smem_set((const void*)vv::k_irfftl<float, float, M>, optin, lowest, e);
+        VV_SETL(512) VV_SETL(1024) VV_SETL(2048)
+#undef VV_SETL
+#define VV_SETT(R, A)                                                \
+    smem_set((const void*)vv::k_tridiagl<R, A, 8>, optin, lowest, e);  \
+    smem_set((const void*)vv::k_tridiagl<R, A, 16>, optin, lowest, e);
+        VV_SETT(double, false) VV_SETT(double, true) VV_SETT(float, false)
+#undef VV_SETT
+#define VV_SETJ1(M)                                                          \
+    smem_set((const void*)vv::k_rfftj1<double, double, M>, optin, lowest, e);  \
+    smem_set((const void*)vv::k_rfftj1<double, float, M>, optin, lowest, e);   \
+    smem_set((const void*)vv::k_rfftj1<float, float, M>, optin, lowest, e);    \
+    smem_set((const void*)vv::k_irfftj1<double, double, M>, optin, lowest, e); \
+    smem_set((const void*)vv::k_irfftj1<float, float, M>, optin, lowest, e);
+        VV_SETJ1(32) VV_SETJ1(64) VV_SETJ1(128) VV_SETJ1(256)
+#undef VV_SETJ1
         smem_set((const void*)vv::k_b_moments_poisson, optin, lowest, e);
         smem_set((const void*)vv::k_adj_poisson, optin, lowest, e);
 #define VV_SET_MARCH(S)                                                              \
@@ -650,6 +677,135 @@ int raise_smem_limits(int* limit_out) {
     return VV_OK;
 }
 
+// ---- v-major preconditioner (vv_pcl.cuh) -------------------------------------
+bool vmaj_ok(const vv_ctx* c) { return c->pow2 && c->M >= 32 && c->M <= 2048; }
+
+template <typename TI, typename R>
+int launch_rfftl(vv_ctx* c, const TI* X, typename Cplx<R>::type* spec, const vv::PcParams& p) {
+    const size_t csz = sizeof(typename Cplx<R>::type);
+#define VV_L(M_)                                                                                              \
+    case M_:                                                                                                  \
+        vv::k_rfftl<TI, R, M_><<<(c->nv + vv::fl_rows(M_) - 1) / vv::fl_rows(M_), vv::FL_THREADS,            \
+                                 vv::fl_smem(M_, csz), c->st>>>(X, spec, p);                                  \
+        break;
+#define VV_J(M_)                                                                                              \
+    case M_:                                                                                                  \
+        vv::k_rfftj1<TI, R, M_><<<(c->nv + vv::fj_rows_of(M_) - 1) / vv::fj_rows_of(M_), vv::FJ_THREADS,      \
+                                  (size_t)vv::fj_slots_of(M_) * csz, c->st>>>(X, spec, p);                    \
+        break;
+    switch (c->M) {
+        VV_J(32) VV_J(64) VV_J(128) VV_J(256) VV_L(512) VV_L(1024) VV_L(2048)
+        default: return VV_ERR_UNSUPPORTED;
+    }
+#undef VV_L
+#undef VV_J
+    CKL(c);
+    return VV_OK;
+}
+
+template <typename R, typename TO>
+int launch_irfftl(vv_ctx* c, const typename Cplx<R>::type* spec, TO* Y, const vv::PcParams& p) {
+    const size_t csz = sizeof(typename Cplx<R>::type);
+#define VV_L(M_)                                                                                              \
+    case M_:                                                                                                  \
+        vv::k_irfftl<R, TO, M_><<<(c->nv + vv::fl_rows(M_) - 1) / vv::fl_rows(M_), vv::FL_THREADS,           \
+                                  vv::fl_smem(M_, csz), c->st>>>(spec, Y, p);                                 \
+        break;
+#define VV_J(M_)                                                                                              \
+    case M_:                                                                                                  \
+        vv::k_irfftj1<R, TO, M_><<<(c->nv + vv::fj_rows_of(M_) - 1) / vv::fj_rows_of(M_), vv::FJ_THREADS,     \
+                                   (size_t)vv::fj_slots_of(M_) * csz, c->st>>>(spec, Y, p);                   \
+        break;
+    switch (c->M) {
+        VV_J(32) VV_J(64) VV_J(128) VV_J(256) VV_L(512) VV_L(1024) VV_L(2048)
+        default: return VV_ERR_UNSUPPORTED;
+    }
+#undef VV_L
+#undef VV_J
+    CKL(c);
+    return VV_OK;
+}
+
+// P^-1 (ADJ: P^-T) through the v-major stages, in the context's GMRES precision
+template <typename TI, typename R, typename TO, bool ADJ>
+int pcl_apply_t(vv_ctx* c, const TI* X, TO* Y, const int* yidx, int yoff) {
+    constexpr bool D = std::is_same<R, double>::value;
+    using C2 = typename Cplx<R>::type;
+    vv::PcParams p = pcparams(c);
+    C2* spec = D ? reinterpret_cast<C2*>(c->spec) : reinterpret_cast<C2*>(c->spec32);
+    C2* spec2 = reinterpret_cast<C2*>(c->vm_spec);
+    p.tw = D ? (const void*)c->tw : (const void*)c->tw32;
+    TRY((launch_rfftl<TI, R>(c, X, spec, p)));
+    vv::TriParams t;
+    t.nv = c->nv;
+    t.nmodes = c->nmodes;
+    t.lambda = D ? (const void*)c->lambda : (const void*)c->lambda32;
+    t.alpha = D ? (const void*)c->alpha : (const void*)c->alpha32;
+    t.gamma = D ? (const void*)c->gamma : (const void*)c->gamma32;
+    t.dinv = nullptr;
+    // chunks of 16 rows, of 8 (twice the blocks, more overlap) where those are fewer than the SMs
+    const int tiles = (c->nmodes + 31) / 32, u16 = (vv::TL_WARPS - 2 * c->vm_lev16) * 16;
+    const int u8 = (vv::TL_WARPS - 2 * c->vm_lev8) * 8;
+    const bool small = u8 > 0 && (u16 <= 0 || tiles * ((c->nv + u16 - 1) / u16) < 148);
+    const int un = small ? u8 : u16;
+    const dim3 g((unsigned)tiles, (unsigned)((c->nv + un - 1) / un));
+    const C2* dj = reinterpret_cast<const C2*>(c->vm_dinv);
+    if (small)
+        vv::k_tridiagl<R, ADJ, 8><<<g, 32 * vv::TL_WARPS, vv::tl_smem<R>(8), c->st>>>(spec, spec2, dj, t, c->vm_lev8);
+    else
+        vv::k_tridiagl<R, ADJ, 16><<<g, 32 * vv::TL_WARPS, vv::tl_smem<R>(16), c->st>>>(spec, spec2, dj, t, c->vm_lev16);
+    CKL(c);
+    p.yidx = yidx;
+    p.yoff = yoff;
+    p.ystride = yidx ? c->ncell : 0;
+    return launch_irfftl<R, TO>(c, spec2, Y, p);
+}
+
+// tables of the v-major preconditioner (false: it does not apply to this grid)
+int vmaj_prepare(vv_ctx* c, bool* ok) {
+    *ok = false;
+    if (!vmaj_ok(c) || !c->cl_lf) return VV_OK;
+    // chunks after which every product of the multipliers is negligible (both sweeps)
+    const double tol = c->mixed ? 1e-9 : 1e-18;
+    auto levels = [&](int ch) {
+        for (int lev = 1; 2 * lev < vv::TL_WARPS; ++lev) {
+            const int w = lev * ch;
+            bool fits = true;
+            for (int j = 0; j + w <= c->nv && fits; ++j) {
+                double a = 1.0, b = 1.0;
+                for (int q = 0; q < w; ++q) {
+                    a *= (*c->cl_lf)[j + q];
+                    b *= (*c->cl_lb)[j + q];
+                }
+                fits = a <= tol * tol && b <= tol * tol;
+            }
+            if (fits) return lev;
+        }
+        return vv::TL_WARPS / 2;   // no useful chunk left
+    };
+    c->vm_lev16 = levels(16);
+    c->vm_lev8 = levels(8);
+    if (vv::TL_WARPS - 2 * c->vm_lev16 <= 0 && vv::TL_WARPS - 2 * c->vm_lev8 <= 0) return VV_OK;
+    const size_t cnt = (size_t)c->nmodes * c->nv, csz = c->mixed ? sizeof(float2) : sizeof(double2);
+    if (!c->vm_dinv) {
+        char* base = nullptr;
+        TRY(dalloc(&base, 2 * cnt * csz + 256));
+        c->vm_dinv = base;
+        c->vm_spec = base + ((cnt * csz + 255) & ~(size_t)255);
+        const unsigned g = (unsigned)((cnt + 255) / 256);
+        if (c->mixed) vv::k_modes_to_vmajor<float2><<<g, 256, 0, c->st>>>(c->dinv32, (float2*)c->vm_dinv, c->nmodes, c->nv);
+        else vv::k_modes_to_vmajor<double2><<<g, 256, 0, c->st>>>(c->dinv, (double2*)c->vm_dinv, c->nmodes, c->nv);
+        CKL(c);
+    }
+    *ok = true;
+    return VV_OK;
+}
+
+void vmaj_release(vv_ctx* c) {
+    if (c->vm_dinv) cudaFree(c->vm_dinv);
+    c->vm_dinv = c->vm_spec = nullptr;
+}
+
 // P^-1 with input type TI, arithmetic R (double: FP64 tables and spectrum,
 // float: the mixed mode's FP32 copies) and output type TO.  Y may be a GMRES
 // basis base pointer with yidx -> the vector index (+yoff).
@@ -657,6 +813,8 @@ template <typename TI, typename R, typename TO>
 int pck_apply_t(vv_ctx* c, const TI* X, TO* Y, const int* yidx = nullptr, int yoff = 0) {
     constexpr bool D = std::is_same<R, double>::value;
     using C2 = typename Cplx<R>::type;
+    if (c->vmaj && D != c->mixed && aligned16(X) && aligned16(Y))
+        return pcl_apply_t<TI, R, TO, false>(c, X, Y, yidx, yoff);
     vv::PcParams p = pcparams(c);
     C2* spec = D ? reinterpret_cast<C2*>(c->spec) : reinterpret_cast<C2*>(c->spec32);
     p.tw = D ? (const void*)c->tw : (const void*)c->tw32;
@@ -804,6 +962,8 @@ int pcT_apply(vv_ctx* c, const double* X, double* Y, const int* yidx = nullptr, 
         if (yidx) return VV_ERR_UNSUPPORTED;
         return copy_d(c, Y, X, c->ncell);
     }
+    if (c->vmaj && !c->mixed && aligned16(X) && aligned16(Y))
+        return pcl_apply_t<double, double, double, true>(c, X, Y, yidx, yoff);
     vv::PcParams p = pcparams(c);
     p.tw = c->tw;
     const unsigned rows = (unsigned)((c->nv + c->pcR - 1) / c->pcR);
@@ -1355,13 +1515,13 @@ bool same_state(const vv_state& a, const vv_state& b) { return std::memcmp(&a, &
 // scratch buffers (CUDA events, a few launches each) and keeps the fastest:
 // FFT kind x rows per CTA x tridiagonal kind for the preconditioner in the
 // GMRES precision, and the bracket tile shape.  Results are cached per
-// (nx, nv, precision, time derivative) for the life of the process.
+// (nx, nv, precision, time derivative, preconditioner) for the life of the process.
 struct TuneResult {
-    int fft_kind, pcR, tri_kind, narrow, march;
+    int fft_kind, pcR, tri_kind, narrow, march, vmaj;
 };
 
-std::vector<std::pair<std::array<int, 4>, TuneResult>>& tune_cache() {
-    static std::vector<std::pair<std::array<int, 4>, TuneResult>> cache;
+std::vector<std::pair<std::array<int, 5>, TuneResult>>& tune_cache() {
+    static std::vector<std::pair<std::array<int, 5>, TuneResult>> cache;
     return cache;
 }
 
@@ -1385,7 +1545,7 @@ int time_it(vv_ctx* c, F fn, int reps, float* ms) {
 }
 
 int autotune(vv_ctx* c) {
-    const std::array<int, 4> key = {c->nx, c->nv, c->mixed ? 1 : 0, c->avg};
+    const std::array<int, 5> key = {c->nx, c->nv, c->mixed ? 1 : 0, c->avg, c->g.preconditioner};
     for (auto& kv : tune_cache())
         if (kv.first == key) {
             c->fft_kind = kv.second.fft_kind;
@@ -1393,12 +1553,17 @@ int autotune(vv_ctx* c) {
             c->tri_kind = kv.second.tri_kind;
             c->narrow_bracket = kv.second.narrow;
             c->march = kv.second.march;
+            if (kv.second.vmaj && c->g.preconditioner == VV_PC_TENSOR_KINETIC) {
+                bool ok = false;
+                TRY(vmaj_prepare(c, &ok));
+                c->vmaj = ok ? 1 : 0;
+            }
             return VV_OK;
         }
     const size_t n = c->ncell;
     CK(cudaMemsetAsync(c->tmp, 0, n * sizeof(double), c->st));
     if (c->mixed) CK(cudaMemsetAsync(c->tmp32, 0, n * sizeof(float), c->st));
-    TuneResult best{c->fft_kind, c->pcR, c->tri_kind, 0, 0};
+    TuneResult best{c->fft_kind, c->pcR, c->tri_kind, 0, 0, 0};
     float best_ms = 1e30f;
     // FP64 complex size also in the mixed mode: the FP64 entry points
     // (vv_pc_apply) share the tuned rows-per-CTA
@@ -1419,7 +1584,7 @@ int autotune(vv_ctx* c) {
                 TRY(r);
                 if (ms < best_ms) {
                     best_ms = ms;
-                    best = {kind, R, tk, 0, 0};
+                    best = {kind, R, tk, 0, 0, 0};
                 }
             }
         }
@@ -1427,6 +1592,23 @@ int autotune(vv_ctx* c) {
     c->fft_kind = best.fft_kind;
     c->pcR = best.pcR;
     c->tri_kind = best.tri_kind;
+    // the v-major stages on grids of 64 K cells and more (below, every variant is at launch latency)
+    if (c->g.preconditioner == VV_PC_TENSOR_KINETIC && c->ncell >= 65536) {
+        bool ok = false;
+        TRY(vmaj_prepare(c, &ok));
+        if (ok) {
+            c->vmaj = 1;
+            float ms = 0.f;
+            TRY(c->mixed ? time_it(c, [&]() { return pc_apply_t<float, float, float>(c, c->tmp32, c->bvec32); }, 5, &ms)
+                         : time_it(c, [&]() { return pc_apply(c, c->tmp, c->bvec); }, 5, &ms));
+            if (ms < best_ms) best.vmaj = 1;
+            else {
+                c->vmaj = 0;
+                CK(cudaStreamSynchronize(c->st));
+                vmaj_release(c);
+            }
+        }
+    }
     if (c->nx % vv::WX == 0) {
         float t_wide = 0.f, t_narrow = 0.f;
         for (int nb = 0; nb <= 1; ++nb) {
@@ -1481,17 +1663,23 @@ int apply_shape(vv_ctx* c, const char* spec) {
     const int n = sscanf(spec, "%d,%d,%d,%d,%d", &v[0], &v[1], &v[2], &v[3], &v[4]);
     if (n < 4) return fail(VV_ERR_ARG, "VV_SHAPE=\"%s\": expected fft,R,tri,narrow[,march]", spec);
     const int kind = v[0], R = v[1], tk = v[2], nb = v[3], mw = v[4];
-    if (kind < 0 || kind > 2 || ((kind == 0 || kind == 1) && !c->pow2) || (kind == 1 && !four_step_ok(c->M)))
+    if (kind == 3 && c->g.preconditioner == VV_PC_TENSOR_KINETIC) {   // v-major stages (radix-2 FFTs and tri where
+        bool ok = false;                                              // the other precision is asked for)
+        TRY(vmaj_prepare(c, &ok));
+        if (!ok) return fail(VV_ERR_ARG, "VV_SHAPE: the v-major preconditioner does not fit nx %d", c->nx);
+        c->vmaj = 1;
+    }
+    if (kind < 0 || kind > 3 || ((kind == 0 || kind == 1) && !c->pow2) || (kind == 1 && !four_step_ok(c->M)))
         return fail(VV_ERR_ARG, "VV_SHAPE: FFT kind %d does not fit nx %d", kind, c->nx);
     if (R != 1 && R != 2 && R != 4 && R != 8)
         return fail(VV_ERR_ARG, "VV_SHAPE: rows per CTA %d not in {1, 2, 4, 8}", R);
-    if (kind < 2 && fft_smem(kind, c->M, R, sizeof(double2), true) > (size_t)c->smem_limit)
+    if (kind != 2 && fft_smem(kind == 3 ? 0 : kind, c->M, R, sizeof(double2), true) > (size_t)c->smem_limit)
         return fail(VV_ERR_ARG, "VV_SHAPE: %d FFT rows per CTA need more shared memory than the limit", R);
     if (tk != 0 && tk != 1) return fail(VV_ERR_ARG, "VV_SHAPE: tridiagonal kind %d not in {0, 1}", tk);
     if (nb != 0 && nb != 1) return fail(VV_ERR_ARG, "VV_SHAPE: narrow flag %d not in {0, 1}", nb);
     if (mw != 0 && ((mw != 128 && mw != 256) || c->nx % mw != 0))
         return fail(VV_ERR_ARG, "VV_SHAPE: marching strip width %d does not fit nx %d", mw, c->nx);
-    c->fft_kind = kind;
+    c->fft_kind = kind == 3 ? 0 : kind;
     c->pcR = kind == 2 ? 1 : R;
     c->tri_kind = tk;
     c->narrow_bracket = nb;
@@ -1935,7 +2123,6 @@ int vv_create(const vv_grid* grid, vv_ctx** out) {
     }
     std::vector<double2> dinv((size_t)nm * nv);
     std::vector<double2> lam2(nm);
-    const bool covers = cl_covers(c);
     bool piv = false;
     for (int k = 0; k < nm; ++k) {
         const cd L = lam[k];
@@ -2114,7 +2301,7 @@ int vv_create(const vv_grid* grid, vv_ctx** out) {
         const char* e = getenv("VV_MARCH");   // fixed strip width (tests, profiling); the autotuner may override
         if (e) c->march = atoi(e);
     }
-    if (covers) {
+    if (g.preconditioner == VV_PC_TENSOR_KINETIC) {
         // |l_j| = |lambda alpha_j / U_{j-1}|, |m_j| = |lambda gamma_j / U_j|
         std::vector<double> mult(nv, 0.0);   // max over the modes of |lambda / U_j|^2
         for (int k = 0; k < nm; ++k) {
@@ -2128,6 +2315,8 @@ int vv_create(const vv_grid* grid, vv_ctx** out) {
             if (j > 0) (*c->cl_lf)[j] = alpha[j] * alpha[j] * mult[j - 1];
             if (j + 1 < nv) (*c->cl_lb)[j] = gamma[j] * gamma[j] * mult[j];
         }
+    }
+    if (cl_covers(c)) {
         // the circulant inverse of the Laplacian on mean-free profiles, symmetric:
         // green_d = (1/nx) sum_k cos(2 pi k d / nx) / symbol_k
         std::vector<double> green(nx), inv(nx / 2 + 1);
@@ -2636,7 +2825,7 @@ int vv_time_kernel(vv_ctx* c, int which, int reps, double* avg_ms) {
 
 int vv_kernel_shape(vv_ctx* c, int32_t* shape) {
     if (!c || !shape) return VV_ERR_ARG;
-    shape[0] = c->fft_kind;
+    shape[0] = c->vmaj ? 3 : c->fft_kind;
     shape[1] = c->pcR;
     shape[2] = c->tri_kind;
     shape[3] = c->narrow_bracket;
@@ -3347,7 +3536,7 @@ int cl_batch_build(vv_batch* b) {
     for (int i = 0; i < n; ++i) {
         vv_ctx* c = b->ctx[i];
         vv::ClShape t{};
-        if (c->cl_lf)
+        if (cl_covers(c))
             for (int ctas = cl_batch_ctas(c); ctas <= vv::CL_MAXC && !t.ctas; ctas *= 2) {
                 t = vv::cl_shape(c->nx, c->nv, c->pow2, ctas, c->mixed ? 4 : 8, vv::cl_smem_limit(c->mixed));
                 if (t.ctas && vv::cl_resident(c->mixed, t.fam, t.ctas, t.smem) < 1) t = vv::ClShape{};
