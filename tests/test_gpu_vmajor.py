@@ -1,0 +1,86 @@
+"""The v-major preconditioner of one grid (vv_pcl.cuh) and the Gram-Schmidt passes at the edges of their tiles."""
+
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+from oracle import vlasov_oracle as vo  # noqa: E402
+
+
+@pytest.fixture(scope="module", autouse=True)
+def _cuda():
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+
+
+# every row length (two and three passes), lines shorter than a chunk, ending inside one and
+# longer than a block's rows; odd row counts leave a block of rows part full
+@pytest.mark.parametrize("nx,nv", [(64, 2053), (64, 16), (128, 193), (256, 385), (512, 97), (1024, 67), (2048, 35),
+                                   (4096, 19), (1024, 5)])
+def test_vmajor_preconditioner_matches_oracle(monkeypatch, nx, nv):
+    """1e-12 relative, as every variant of the preconditioner (carries cut off below 1e-18)."""
+    from vivlasov1d_b200.solver import Grid, TensorProductPreconditioner
+    monkeypatch.setenv("VV_SHAPE", "3,1,0,0,0")
+    og = vo.Grid(nx, nv, 4 * np.pi, 8.0, ht=0.05)
+    grid = Grid(nx, nv, 4 * np.pi, 8.0, ht=0.05)
+    x = np.random.default_rng(nx + nv).standard_normal((nx, nv))
+    pc = TensorProductPreconditioner.create("tensor_kinetic", grid=grid)
+    assert pc.ctx.kernel_shape()[0] == 3
+    X, Y = torch.from_numpy(vo.to_flat(x)).cuda(), grid.field()
+    pc.tensorProduct(X, Y)
+    want = vo.TensorKineticPreconditioner(og).apply(x)
+    got = vo.from_flat(Y.cpu().numpy())
+    assert np.abs(got - want).max() <= 1e-12 * np.abs(want).max()
+    pc.tensorProduct(X, X)     # in place
+    assert torch.equal(X, Y)
+
+
+@pytest.mark.parametrize("nx,nv", [(128, 300), (1024, 80)])
+def test_vmajor_mixed_step_and_adjoint(monkeypatch, nx, nv):
+    """A mixed step and the transposed solve through the v-major stages against the other variants: f within the
+    residual ball (2 ht atol), the adjoint within its GMRES tolerance."""
+    from vivlasov1d_b200.adjoint import Adjoint
+    from vivlasov1d_b200.run import Run
+    cfg = {"grid": {"nx": nx, "nv": nv, "L": 4 * np.pi, "vmin": -8.0, "vmax": 8.0, "ht": 0.05, "nt": 1},
+           "solver": {"method": "matrixfree", "poisson_bracket": "ArakawaJ4", "preconditioner_type": "tensor",
+                      "preconditioner_scheme": "tensor_kinetic", "petsc_ksp_rtol": 1e-6, "petsc_snes_atol": 1e-10},
+           "initial_data": {"charge": -1.0}}
+    og = vo.Grid(nx, nv, 4 * np.pi, 8.0, -8.0, ht=0.05)
+    f0 = torch.from_numpy(vo.to_flat(vo.initialise_distribution_function(og, vo.f0_twostream(0.05, 0.5))))
+    w = torch.from_numpy(np.random.default_rng(1).standard_normal((nv, nx))).cuda()
+    outs = []
+    for shape in ("3,1,0,0,0", "0,1,0,0,0"):
+        monkeypatch.setenv("VV_SHAPE", shape)
+        mixed, run = Run(cfg, f0=f0, precision="mixed"), Run(cfg, f0=f0)
+        f = run.fc.clone()
+        mixed.step()
+        run.step()
+        outs.append((mixed.fc, run.fc, Adjoint(run).step(run.fc, f, w)))
+    (m1, f1, g1), (m2, f2, g2) = outs
+    bound = 2 * 2 * 0.05 * 1e-10
+    assert float((m1 - m2).norm()) <= bound and float((f1 - f2).norm()) <= bound
+    assert float((g1 - g2).norm()) <= 1e-8 * float(g2.norm())
+
+
+@pytest.mark.parametrize("nx,nv,restart", [(15, 17, 30), (64, 33, 64), (33, 4999, 30), (256, 2400, 31)])
+def test_gram_schmidt_passes(monkeypatch, nx, nv, restart):
+    """The multi-kernel GMRES on grids whose vectors are and are not 16-byte aligned, of few and of many tiles, with
+    a solution vector that is not 16-byte aligned: the residual it reports is the residual it leaves."""
+    from vivlasov1d_b200.solver import Grid, PETScVlasovSolver
+    monkeypatch.setenv("VV_CLUSTER", "0")
+    grid = Grid(nx, nv, 4 * np.pi, 8.0, ht=0.05)
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    h1 = 0.1 * torch.rand(nx, generator=gen, dtype=torch.float64, device="cuda")
+    cfg = {"poisson_bracket": "arakawaj4", "preconditioner": "tensor_kinetic"}
+    s = PETScVlasovSolver(cfg, None, None, grid, None, h1, h1, None, None, None, restart=restart)
+    s.update_previous()
+    b = torch.rand((nv, nx), generator=gen, dtype=torch.float64, device="cuda") - 0.5
+    x = torch.empty(nx * nv + 1, dtype=torch.float64, device="cuda")[1:].view(nv, nx)
+    its, reason, rnorm = s.gmres(b, x, rtol=1e-9, max_it=500)
+    # the last two grids reach 500 iterations first (a rough profile), the others the tolerance
+    assert (reason == 2 and rnorm <= 1e-9 * float(b.norm())) or (reason == -3 and its == 500)
+    y = grid.field()
+    s.jacobian(x.clone(), y)
+    assert float((b - y).norm()) <= 1.01 * rnorm + 1e-9 * float(b.norm())

@@ -88,6 +88,7 @@ __global__ void k_adj_coef(AdjParams p, const double* __restrict__ h0, const dou
 }
 
 constexpr int ADJ_TX = 32, ADJ_TY = 8;
+constexpr int ADJ_SEG = 16;   // v rows of a block: two per thread, so that a medium grid fills the GPU
 
 // out = y/ht + 1/2 J_H^T y, and the v-sums of z = J_Fbar^T y per segment:
 // zpart[s * nx + i] (segments of `seg` rows).  Grid (ceil(nx/32), S).
@@ -137,6 +138,7 @@ k_adj_poisson(const double* __restrict__ zpart, int S, double* __restrict__ zbuf
               PoissonParams po) {
     for (int i = threadIdx.x; i < po.nx; i += blockDim.x) {
         double t = 0.0;
+#pragma unroll 8
         for (int s = 0; s < S; ++s) t += zpart[(size_t)s * po.nx + i];
         zbuf[i] = t;
     }

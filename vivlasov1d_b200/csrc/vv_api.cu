@@ -941,11 +941,12 @@ vv::AdjParams adjparams(const vv_ctx* c) {
 // Y = A^T X (X may be a basis base pointer with xidx)
 int adj_apply(vv_ctx* c, const double* X, const int* xidx, double* Y) {
     const vv::AdjParams p = adjparams(c);
-    dim3 grid((c->nx + vv::ADJ_TX - 1) / vv::ADJ_TX, c->mom_S);
-    vv::k_adj_apply<<<grid, dim3(vv::ADJ_TX, vv::ADJ_TY), 0, c->st>>>(p, c->adj_cH, c->adj_cF, X, xidx, Y, c->mom_seg,
+    const int S = (c->nv + vv::ADJ_SEG - 1) / vv::ADJ_SEG;
+    dim3 grid((c->nx + vv::ADJ_TX - 1) / vv::ADJ_TX, S);
+    vv::k_adj_apply<<<grid, dim3(vv::ADJ_TX, vv::ADJ_TY), 0, c->st>>>(p, c->adj_cH, c->adj_cF, X, xidx, Y, vv::ADJ_SEG,
                                                                       c->adj_zpart);
     CKL(c);
-    vv::k_adj_poisson<<<1, vv::POIS_THREADS, c->smem_pois, c->st>>>(c->adj_zpart, c->mom_S, c->adj_zbuf, c->adj_q,
+    vv::k_adj_poisson<<<1, vv::POIS_THREADS, c->smem_pois, c->st>>>(c->adj_zpart, S, c->adj_zbuf, c->adj_q,
                                                                     pparams(c));
     CKL(c);
     vv::k_adj_bcast<<<grid1d(c->ncell, 256), 256, 0, c->st>>>(p, c->adj_q, Y);
@@ -1171,14 +1172,38 @@ int gm_cycle_start(vv_ctx* c) {
     return VV_OK;
 }
 
+// launch(values per item, blocks): 16-byte items where the vectors (and x) are
+// aligned; at most 592 blocks (the partials' width), each with the same number of
+// tiles.  One item of a thread and four vectors in flight: two steps of 1024 x
+// 2048 mixed 121 ms; four items and two vectors, in whole tiles, 143 ms.  The
+// averaged time derivatives keep single values and 2048 cells per block: their
+// Jacobian is nearly singular, so round-off decides whether a step's last solves
+// converge, and the order of these sums is the one their behaviour was measured in.
+template <typename T, typename F>
+int gs_launch(vv_ctx* c, const T* x, F launch) {
+    constexpr int VN = 16 / (int)sizeof(T);
+    if (c->avg != vv::AVG_POINT || c->ncell % VN != 0 || !aligned16(x)) {
+        launch(std::integral_constant<int, 1>{}, (unsigned)c->npart);
+    } else {
+        const size_t tiles = (c->ncell / VN + vv::RED_THREADS - 1) / vv::RED_THREADS;
+        const size_t rounds = (tiles + c->npart_max - 1) / c->npart_max;
+        launch(std::integral_constant<int, VN>{}, (unsigned)((tiles + rounds - 1) / rounds));
+    }
+    CKL(c);
+    return VV_OK;
+}
+
 template <typename T>
 int gm_arnoldi(vv_ctx* c) {
     T* V = Buf<T>::V(c);
     TRY(apply_operator_state<T>(c));
-    vv::k_gm_mdot<T><<<c->npart, vv::RED_THREADS, 0, c->st>>>(c->ds, V, c->ncell, c->ncell, c->part, c->npart_max);
-    CKL(c);
-    vv::k_gm_maxpy<T><<<c->npart, vv::RED_THREADS, 0, c->st>>>(c->ds, V, c->ncell, c->ncell, c->part);
-    CKL(c);
+    TRY(gs_launch<T>(c, V, [&](auto vn, unsigned g) {
+        vv::k_gm_mdot<T, decltype(vn)::value><<<g, vv::RED_THREADS, 0, c->st>>>(c->ds, V, c->ncell, c->ncell, c->part,
+                                                                         c->npart_max);
+    }));
+    TRY(gs_launch<T>(c, V, [&](auto vn, unsigned g) {
+        vv::k_gm_maxpy<T, decltype(vn)::value><<<g, vv::RED_THREADS, 0, c->st>>>(c->ds, V, c->ncell, c->ncell, c->part);
+    }));
     vv::k_gm_scale<T><<<grid1d(c->ncell, 256), 256, 0, c->st>>>(c->ds, V, c->ncell, c->ncell);
     CKL(c);
     return VV_OK;
@@ -1186,9 +1211,10 @@ int gm_arnoldi(vv_ctx* c) {
 
 template <typename T>
 int gm_finish(vv_ctx* c, T* x) {
-    vv::k_gm_finish<T><<<c->npart, vv::RED_THREADS, 0, c->st>>>(c->ds, Buf<T>::V(c), c->ncell, x, c->ncell);
-    CKL(c);
-    return VV_OK;
+    return gs_launch<T>(c, x, [&](auto vn, unsigned g) {
+        vv::k_gm_finish<T, decltype(vn)::value><<<g, vv::RED_THREADS, 0, c->st>>>(c->ds, Buf<T>::V(c), c->ncell, x,
+                                                                                 c->ncell);
+    });
 }
 
 struct GmHead {
@@ -2580,7 +2606,7 @@ int adj_buffers(vv_ctx* c) {
     int s = VV_OK;
     const size_t nx = c->nx;
     if ((s = dalloc(&c->adj_cH, (size_t)vv::ADJ_NOFF * c->ncell)) || (s = dalloc(&c->adj_cF, (size_t)vv::ADJ_NOFF * c->ncell)) ||
-        (s = dalloc(&c->adj_zpart, (size_t)c->mom_S * nx)) || (s = dalloc(&c->adj_zbuf, nx)) ||
+        (s = dalloc(&c->adj_zpart, (size_t)((c->nv + vv::ADJ_SEG - 1) / vv::ADJ_SEG) * nx)) || (s = dalloc(&c->adj_zbuf, nx)) ||
         (s = dalloc(&c->adj_q, nx)) || (s = dalloc(&c->adj_hprof, nx)) || (s = dalloc(&c->adj_h1a, nx)) ||
         (s = dalloc(&c->adj_h1b, nx)))
         return s;

@@ -10,7 +10,6 @@ namespace vv {
 
 constexpr int RED_THREADS = 256;
 constexpr int MAX_RESTART = 64;
-constexpr int MDOT_CHUNK = 8;
 
 // ---------------------------------------------------------------------------
 // Device-resident solver state: GMRES (PETSc KSP_GMRES arrays: hh = rotated
@@ -229,55 +228,108 @@ __global__ void k_gm_scale(DevState* s, T* __restrict__ V, size_t ldv, size_t n)
     gm_scale_block<T>(s, V, ldv, n, blockIdx.x, gridDim.x);
 }
 
-// hcol_q = <w, V_q>, q = 0..it, w = V[it+1]  (one multi-dot, last CTA reduces)
-template <typename T>
-__device__ __forceinline__ void gm_mdot_block(DevState* s, const T* __restrict__ V, size_t ldv, size_t n,
-                                              double* __restrict__ part, int ld, int bid, int nblk) {
-    static_assert(MDOT_CHUNK <= RED_THREADS / 32, "one warp per dot of a chunk");
-    __shared__ double shc[MDOT_CHUNK][RED_THREADS / 32];
-    const int it = s->it;
-    const int m = it + 1;
-    const T* w = V + (size_t)(it + 1) * ldv;
-    for (int q0 = 0; q0 < m; q0 += MDOT_CHUNK) {
-        double acc[MDOT_CHUNK];
-#pragma unroll
-        for (int c = 0; c < MDOT_CHUNK; ++c) acc[c] = 0.0;
-        const int cnt = min(MDOT_CHUNK, m - q0);
-        for (size_t i = bid * (size_t)RED_THREADS + threadIdx.x; i < n; i += (size_t)nblk * RED_THREADS) {
-            const double wi = (double)w[i];
-#pragma unroll
-            for (int c = 0; c < MDOT_CHUNK; ++c)
-                if (c < cnt) acc[c] += wi * (double)V[(size_t)(q0 + c) * ldv + i];
-        }
-        // block sums of the chunk's dots: warp sums, one barrier, then warp c
-        // adds the warp sums of dot c (the order of block_sum)
-        const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-#pragma unroll
-        for (int c = 0; c < MDOT_CHUNK; ++c) {
-            if (c < cnt) {
-                const double t = warp_sum(acc[c]);
-                if (lane == 0) shc[c][wid] = t;
-            }
-        }
-        __syncthreads();
-        if (wid < cnt) {
-            double r = (lane < RED_THREADS / 32) ? shc[wid][lane] : 0.0;
-            r = warp_sum(r);
-            if (lane == 0) part[(size_t)(q0 + wid) * ld + bid] = r;
-        }
-        __syncthreads();
+// Gram-Schmidt items: VN consecutive values (16 bytes, or one where the
+// vectors are not 16-byte aligned), one per thread and tile, with the loads of
+// GS_Q basis vectors in flight.  The passes stream the basis from HBM or L2;
+// with one value and one vector at a time they ran at the latency of a load per
+// basis vector (256 x 512 FP64 at mean index 15: multi-dot 37 -> 14 us, multi-axpy
+// 61 -> 14; 1024 x 2048 FP32: 46 -> 30 and 87 -> 31 us).
+constexpr int GS_Q = 4;
+template <typename T, int VN> struct GsVec { T v[VN]; };
+template <typename T, int VN> VV_DEV GsVec<T, VN> gs_ld(const T* p) {
+    GsVec<T, VN> o;
+    if constexpr (VN == 1) {
+        o.v[0] = *p;
+    } else if constexpr (VN == 2) {
+        const double2 q = *reinterpret_cast<const double2*>(p);
+        o.v[0] = q.x;
+        o.v[1] = q.y;
+    } else {
+        const float4 q = *reinterpret_cast<const float4*>(p);
+        o.v[0] = q.x;
+        o.v[1] = q.y;
+        o.v[2] = q.z;
+        o.v[3] = q.w;
     }
-    if (!last_block(&s->cnt[1], nblk)) return;
-    const int wid = threadIdx.x >> 5;
-    for (int q = wid; q < m; q += RED_THREADS / 32) {
-        const double t = warp_reduce_parts(part + (size_t)q * ld, nblk);
-        if ((threadIdx.x & 31) == 0) s->hcol[q] = t;
-    }
+    return o;
 }
-template <typename T>
+template <typename T, int VN> VV_DEV void gs_st(T* p, const double (&w)[VN]) {
+    if constexpr (VN == 1) *p = (T)w[0];
+    else if constexpr (VN == 2) *reinterpret_cast<double2*>(p) = make_double2(w[0], w[1]);
+    else *reinterpret_cast<float4*>(p) = make_float4((float)w[0], (float)w[1], (float)w[2], (float)w[3]);
+}
+
+// hcol_q = <w, V_q>, q = 0..it, w = V[it+1]  (one multi-dot, last CTA reduces)
+template <typename T, int VN>
 __global__ void __launch_bounds__(RED_THREADS)
 k_gm_mdot(DevState* s, const T* __restrict__ V, size_t ldv, size_t n, double* __restrict__ part, int ld) {
-    gm_mdot_block<T>(s, V, ldv, n, part, ld, blockIdx.x, gridDim.x);
+    __shared__ double dots[MAX_RESTART + 2][RED_THREADS / 32];
+    const int m = s->it + 1, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const T* w = V + (size_t)m * ldv;
+    const size_t E = n / VN, tiles = (E + RED_THREADS - 1) / RED_THREADS;
+    // sums of the lanes of GS_Q dots together
+    auto lanes = [&](double (&t)[GS_Q]) {
+#pragma unroll
+        for (int h = 16; h > 0; h >>= 1)
+#pragma unroll
+            for (int u = 0; u < GS_Q; ++u) t[u] += __shfl_xor_sync(0xffffffffu, t[u], h);
+    };
+    if constexpr (VN == 1) {
+        // one sum per thread over all its items
+        for (int q0 = 0; q0 < m; q0 += GS_Q) {
+            double t[GS_Q] = {};
+            for (size_t e = blockIdx.x * (size_t)RED_THREADS + threadIdx.x; e < E; e += (size_t)gridDim.x * RED_THREADS) {
+                const double wi = (double)w[e];
+                T x[GS_Q];
+#pragma unroll
+                for (int u = 0; u < GS_Q; ++u) x[u] = V[(size_t)min(q0 + u, m - 1) * ldv + e];
+#pragma unroll
+                for (int u = 0; u < GS_Q; ++u) t[u] += wi * (double)x[u];
+            }
+            lanes(t);
+            if (lane == 0) {
+#pragma unroll
+                for (int u = 0; u < GS_Q; ++u)
+                    if (q0 + u < m) dots[q0 + u][wid] = t[u];
+            }
+        }
+    } else {
+        for (size_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+            const size_t e = tile * RED_THREADS + threadIdx.x, o = (e < E ? e : E - 1) * VN;
+            const GsVec<T, VN> x0 = gs_ld<T, VN>(w + o);
+            double wv[VN];
+#pragma unroll
+            for (int i = 0; i < VN; ++i) wv[i] = e < E ? (double)x0.v[i] : 0.0;
+            for (int q0 = 0; q0 < m; q0 += GS_Q) {
+                GsVec<T, VN> x[GS_Q];
+#pragma unroll
+                for (int u = 0; u < GS_Q; ++u) x[u] = gs_ld<T, VN>(V + (size_t)min(q0 + u, m - 1) * ldv + o);
+                double t[GS_Q];
+#pragma unroll
+                for (int u = 0; u < GS_Q; ++u) {
+                    t[u] = 0.0;
+#pragma unroll
+                    for (int i = 0; i < VN; ++i) t[u] += wv[i] * (double)x[u].v[i];
+                }
+                lanes(t);
+                if (lane == 0) {
+#pragma unroll
+                    for (int u = 0; u < GS_Q; ++u)
+                        if (q0 + u < m) dots[q0 + u][wid] = (tile == blockIdx.x ? 0.0 : dots[q0 + u][wid]) + t[u];
+                }
+            }
+        }
+    }
+    __syncthreads();
+    for (int q = wid; q < m; q += RED_THREADS / 32) {
+        const double t = warp_sum(lane < RED_THREADS / 32 ? dots[q][lane] : 0.0);
+        if (lane == 0) part[(size_t)q * ld + blockIdx.x] = t;
+    }
+    if (!last_block(&s->cnt[1], gridDim.x)) return;
+    for (int q = wid; q < m; q += RED_THREADS / 32) {
+        const double t = warp_reduce_parts(part + (size_t)q * ld, gridDim.x);
+        if (lane == 0) s->hcol[q] = t;
+    }
 }
 
 // Arnoldi bookkeeping after tt = ||w|| (KSPGMRESCycle + UpdateHessenberg)
@@ -339,36 +391,62 @@ VV_DEV void gm_arnoldi(DevState* s, double tt, const double* hcol, const double*
 }
 VV_DEV void gm_arnoldi(DevState* s, double tt) { gm_arnoldi(s, tt, s->hcol, s->cc, s->ss); }
 
+// w += sum_q cf_q V_q, q < m, over a block's items: init(o, w) and out(o, w) at
+// the item's offset
+template <typename T, int VN, typename Init, typename Out>
+__device__ __forceinline__ void gs_axpy_tiles(const T* __restrict__ V, size_t ldv, size_t n, int m, const double* cf,
+                                              Init init, Out out) {
+    const size_t E = n / VN;
+    for (size_t e = blockIdx.x * (size_t)RED_THREADS + threadIdx.x; e < E; e += (size_t)gridDim.x * RED_THREADS) {
+        const size_t o = e * VN;
+        double w[VN];
+        init(o, w);
+        for (int q0 = 0; q0 < m; q0 += GS_Q) {
+            GsVec<T, VN> x[GS_Q];
+#pragma unroll
+            for (int u = 0; u < GS_Q; ++u) x[u] = gs_ld<T, VN>(V + (size_t)min(q0 + u, m - 1) * ldv + o);
+#pragma unroll
+            for (int u = 0; u < GS_Q; ++u)
+                if (q0 + u < m) {
+                    const double c = cf[q0 + u];
+#pragma unroll
+                    for (int i = 0; i < VN; ++i) w[i] += c * (double)x[u].v[i];
+                }
+        }
+        out(o, w);
+    }
+}
+
 // w += sum_q (-hcol_q) V_q and ||w||^2 (classical Gram-Schmidt update,
 // VecMAXPY with lhh = -<w,v>); the last CTA finishes the Arnoldi step.
-template <typename T>
-__device__ __forceinline__ void gm_maxpy_block(DevState* s, T* __restrict__ V, size_t ldv, size_t n,
-                                               double* __restrict__ part, int bid, int nblk) {
+template <typename T, int VN>
+__global__ void __launch_bounds__(RED_THREADS)
+k_gm_maxpy(DevState* s, T* __restrict__ V, size_t ldv, size_t n, double* __restrict__ part) {
     __shared__ double sh[RED_THREADS / 32];
     __shared__ double cf[MAX_RESTART + 2];
-    const int it = s->it;
-    const int m = it + 1;
-    T* w = V + (size_t)(it + 1) * ldv;
+    const int m = s->it + 1;
+    T* w = V + (size_t)m * ldv;
     for (int q = threadIdx.x; q < m; q += RED_THREADS) cf[q] = -s->hcol[q];
     __syncthreads();
     double acc = 0.0;
-    for (size_t i = bid * (size_t)RED_THREADS + threadIdx.x; i < n; i += (size_t)nblk * RED_THREADS) {
-        double wi = (double)w[i];
-        for (int q = 0; q < m; ++q) wi += cf[q] * (double)V[(size_t)q * ldv + i];
-        w[i] = (T)wi;
-        acc += wi * wi;
-    }
+    gs_axpy_tiles<T, VN>(
+        V, ldv, n, m, cf,
+        [&](size_t o, double (&wv)[VN]) {
+            const GsVec<T, VN> x = gs_ld<T, VN>(w + o);
+#pragma unroll
+            for (int i = 0; i < VN; ++i) wv[i] = (double)x.v[i];
+        },
+        [&](size_t o, const double (&wv)[VN]) {
+            gs_st<T, VN>(w + o, wv);
+#pragma unroll
+            for (int i = 0; i < VN; ++i) acc += wv[i] * wv[i];
+        });
     const double t = block_sum(acc, sh);
-    if (threadIdx.x == 0) part[bid] = t;
-    if (!last_block(&s->cnt[2], nblk)) return;
+    if (threadIdx.x == 0) part[blockIdx.x] = t;
+    if (!last_block(&s->cnt[2], gridDim.x)) return;
     if (threadIdx.x >= 32) return;
-    const double ss2 = warp_reduce_parts(part, nblk);
+    const double ss2 = warp_reduce_parts(part, gridDim.x);
     if (threadIdx.x == 0) gm_arnoldi(s, sqrt(ss2));
-}
-template <typename T>
-__global__ void __launch_bounds__(RED_THREADS)
-k_gm_maxpy(DevState* s, T* __restrict__ V, size_t ldv, size_t n, double* __restrict__ part) {
-    gm_maxpy_block<T>(s, V, ldv, n, part, blockIdx.x, gridDim.x);
 }
 
 // KSPGMRESBuildSoln: every CTA solves the small triangular system (thread 0,
@@ -412,27 +490,24 @@ VV_DEV void gm_finish_state(DevState* s, int npad, int breakdown) {
     set_cond(s->h_gm_first, 0u);
 }
 
-template <typename T>
-__device__ __forceinline__ void gm_finish_block(DevState* s, const T* __restrict__ V, size_t ldv, T* __restrict__ x,
-                                                size_t n, int bid, int nblk) {
+template <typename T, int VN>
+__global__ void __launch_bounds__(RED_THREADS)
+k_gm_finish(DevState* s, const T* __restrict__ V, size_t ldv, T* __restrict__ x, size_t n) {
     __shared__ double nrs[MAX_RESTART + 1];
     __shared__ int npad, breakdown;
     if (threadIdx.x == 0) gm_backsolve(s, nrs, &npad, &breakdown);
     __syncthreads();
     const int m = npad;
-    if (m > 0) {
-        for (size_t i = bid * (size_t)RED_THREADS + threadIdx.x; i < n; i += (size_t)nblk * RED_THREADS) {
-            double xi = (double)x[i];
-            for (int q = 0; q < m; ++q) xi += nrs[q] * (double)V[(size_t)q * ldv + i];
-            x[i] = (T)xi;
-        }
-    }
-    if (bid == 0 && threadIdx.x == 0) gm_finish_state(s, m, breakdown);
-}
-template <typename T>
-__global__ void __launch_bounds__(RED_THREADS)
-k_gm_finish(DevState* s, const T* __restrict__ V, size_t ldv, T* __restrict__ x, size_t n) {
-    gm_finish_block<T>(s, V, ldv, x, n, blockIdx.x, gridDim.x);
+    if (m > 0)
+        gs_axpy_tiles<T, VN>(
+            V, ldv, n, m, nrs,
+            [&](size_t o, double (&xv)[VN]) {
+                const GsVec<T, VN> v = gs_ld<T, VN>(x + o);
+#pragma unroll
+                for (int i = 0; i < VN; ++i) xv[i] = (double)v.v[i];
+            },
+            [&](size_t o, const double (&xv)[VN]) { gs_st<T, VN>(x + o, xv); });
+    if (blockIdx.x == 0 && threadIdx.x == 0) gm_finish_state(s, m, breakdown);
 }
 
 // ----- Picard-loop kernels -------------------------------------------------
