@@ -70,9 +70,12 @@ struct vv_ctx {
     // for n = nv, nv twiddles, transposed field, v spectrum, elimination
     // scratch (FP32 copies in the mixed mode), rows per CTA of the v FFT, phi
     int nmv, pvR;
-    double2 *lamv, *twv, *pv_spec, *pv_scr;
+    double2 *lamv, *twv, *pv_spec;
+    void* pv_tab;   // the factors' storage
+    vv::PotLu<double2> pv_lu;
+    vv::PotLu<float2> pv_lu32;
     double *pv_xt, *phipc;
-    float2 *twv32, *pv_spec32, *pv_scr32;
+    float2 *twv32, *pv_spec32;
     float* pv_xt32;
     cudaStream_t st;      // the caller's stream
     int device;
@@ -848,9 +851,23 @@ int pck_apply_t(vv_ctx* c, const TI* X, TO* Y, const int* yidx = nullptr, int yo
     return launch_irfft<R, TO>(c, spec, Y, p, rows);
 }
 
+// factors of the potential preconditioner from c->phipc
+int pcv_factor(vv_ctx* c) {
+    vv::PotParams q;
+    q.nx = c->nx;
+    q.nmv = c->nmv;
+    q.arak = 0.5 * c->hx_inv * c->hv_inv / 12.;   // TensorProductPotentialFast.pyx:237
+    q.ht_inv = c->ht_inv;
+    q.phi = c->phipc;
+    q.lam = c->lamv;
+    vv::k_pcv_factor<<<(unsigned)((c->nmv + 31) / 32), 32, 0, c->st>>>(c->pv_lu, c->pv_lu32, q);
+    CKL(c);
+    return VV_OK;
+}
+
 // The potential preconditioner: the v transforms as row transforms of the
 // transposed field (radix-2 FFT for a power-of-two nv, else the direct DFT),
-// the x-tridiagonal systems per v mode by elimination with partial pivoting
+// the x-tridiagonal systems per v mode from their factors
 template <typename TI, typename R, typename TO>
 int pcv_apply_t(vv_ctx* c, const TI* X, TO* Y, const int* yidx = nullptr, int yoff = 0) {
     constexpr bool D = std::is_same<R, double>::value;
@@ -858,7 +875,6 @@ int pcv_apply_t(vv_ctx* c, const TI* X, TO* Y, const int* yidx = nullptr, int yo
     const int nx = c->nx, nv = c->nv;
     R* xt = D ? reinterpret_cast<R*>(c->pv_xt) : reinterpret_cast<R*>(c->pv_xt32);
     C2* spec = D ? reinterpret_cast<C2*>(c->pv_spec) : reinterpret_cast<C2*>(c->pv_spec32);
-    C2* scr = D ? reinterpret_cast<C2*>(c->pv_scr) : reinterpret_cast<C2*>(c->pv_scr32);
     const dim3 tb(32, 8);
     vv::k_transpose<TI, R><<<dim3((nx + 31) / 32, (nv + 31) / 32), tb, 0, c->st>>>(X, xt, nv, nx, nullptr, 0, 0);
     CKL(c);
@@ -878,14 +894,9 @@ int pcv_apply_t(vv_ctx* c, const TI* X, TO* Y, const int* yidx = nullptr, int yo
     if (fft) vv::k_rfft_rows<R, R><<<gr, 32 * c->pvR, fft_smem(0, nv / 2, c->pvR, csz, false), c->st>>>(xt, spec, p);
     else vv::k_rdft_rows<R, R><<<gd, vv::DFT_THREADS, rdft_smem(nv, csz), c->st>>>(xt, spec, p);
     CKL(c);
-    vv::PotParams q;
-    q.nx = nx;
-    q.nmv = c->nmv;
-    q.arak = 0.5 * c->hx_inv * c->hv_inv / 12.;   // TensorProductPotentialFast.pyx:237
-    q.ht_inv = c->ht_inv;
-    q.phi = c->phipc;
-    q.lam = c->lamv;
-    vv::k_pcv_solve<R><<<(unsigned)((c->nmv + 63) / 64), 64, 0, c->st>>>(spec, scr, q);
+    const unsigned gm = (unsigned)((c->nmv + 31) / 32);
+    if constexpr (D) vv::k_pcv_solve<double><<<gm, 32, 0, c->st>>>(spec, c->pv_lu, nx, c->nmv);
+    else vv::k_pcv_solve<float><<<gm, 32, 0, c->st>>>(spec, c->pv_lu32, nx, c->nmv);
     CKL(c);
     if (fft) vv::k_irfft_rows<R, R><<<gr, 32 * c->pvR, fft_smem(0, nv / 2, c->pvR, csz, true), c->st>>>(spec, xt, p);
     else vv::k_irdft_rows<R, R><<<gd, vv::DFT_THREADS, irdft_smem(nv, csz), c->st>>>(spec, xt, p);
@@ -1492,7 +1503,10 @@ int step_prologue(vv_ctx* c, vv_state* st) {
     if (st->phih) TRY(copy_d(c, st->phih, st->phi, nx));
     TRY(copy_d(c, c->Fh, st->f, n));
     // update_history -> update_matrices of the potential preconditioner
-    if (c->g.preconditioner == VV_PC_TENSOR_POTENTIAL) TRY(copy_d(c, c->phipc, st->phi, nx));
+    if (c->g.preconditioner == VV_PC_TENSOR_POTENTIAL) {
+        TRY(copy_d(c, c->phipc, st->phi, nx));
+        TRY(pcv_factor(c));
+    }
     // nc -> nh, uc -> uh, ac -> ah (run_base.py:757-760) for the collision operator
     if (c->coll != vv::COLL_NONE) {
         TRY(copy_d(c, c->mom_h, st->n, nx));
@@ -2230,11 +2244,11 @@ int vv_create(const vv_grid* grid, vv_ctx** out) {
         c->pvR = 4;
         while (c->pvR > 1 && fft_smem(0, nv / 2, c->pvR, sizeof(double2), true) > 200 * 1024) c->pvR /= 2;
         if ((s = dalloc(&c->lamv, nmv)) || (s = dalloc(&c->twv, (size_t)nv)) || (s = dalloc(&c->pv_xt, n)) ||
-            (s = dalloc(&c->pv_spec, (size_t)nmv * nx)) || (s = dalloc(&c->pv_scr, (size_t)3 * nmv * nx)) ||
+            (s = dalloc(&c->pv_spec, (size_t)nmv * nx)) ||
+            (s = dalloc((char**)&c->pv_tab, (size_t)nmv * nx * (4 * 16 + (c->mixed ? 4 * 8 : 0) + 1))) ||
             (s = dalloc(&c->phipc, (size_t)nx)) ||
             (c->mixed && ((s = dalloc(&c->twv32, (size_t)nv)) || (s = dalloc(&c->pv_xt32, n)) ||
-                          (s = dalloc(&c->pv_spec32, (size_t)nmv * nx)) ||
-                          (s = dalloc(&c->pv_scr32, (size_t)3 * nmv * nx))))) {
+                          (s = dalloc(&c->pv_spec32, (size_t)nmv * nx))))) {
             vv_destroy(c);
             return s;
         }
@@ -2262,6 +2276,16 @@ int vv_create(const vv_grid* grid, vv_ctx** out) {
             cudaMemset(c->phipc, 0, nx * sizeof(double)) != cudaSuccess) {
             vv_destroy(c);
             return fail_cuda(cudaGetLastError(), "vv_create upload (potential preconditioner)");
+        }
+        const size_t cnt = (size_t)nmv * nx;
+        double2* t = (double2*)c->pv_tab;
+        c->pv_lu = {t, t + cnt, t + 2 * cnt, t + 3 * cnt, nullptr};
+        float2* t32 = (float2*)(t + 4 * cnt);
+        if (c->mixed) c->pv_lu32 = {t32, t32 + cnt, t32 + 2 * cnt, t32 + 3 * cnt, nullptr};
+        c->pv_lu.swap = c->pv_lu32.swap = (unsigned char*)(c->mixed ? t32 + 4 * cnt : t32);
+        if ((s = pcv_factor(c)) != VV_OK) {
+            vv_destroy(c);
+            return s;
         }
     }
     // double bracket: Fave and the inner bracket
@@ -2407,9 +2431,9 @@ int vv_destroy(vv_ctx* c) {
                     c->sym_inv, c->ds, c->V32, c->tmp32, c->bvec32, c->delta32, c->alpha32, c->gamma32,
                     c->spec32, c->tw32, c->lambda32, c->dinv32, c->adj_cH, c->adj_cF, c->adj_zpart,
                     c->adj_zbuf, c->adj_q, c->adj_hprof, c->adj_h1a, c->adj_h1b, c->lamv, c->twv, c->pv_spec,
-                    c->pv_scr, c->pv_xt, c->phipc, c->twv32, c->pv_spec32, c->pv_scr32, c->pv_xt32,
+                    c->pv_tab, c->pv_xt, c->phipc, c->twv32, c->pv_spec32, c->pv_xt32,
                     c->mom_p, c->mom_h, c->db_fave, c->db_b, c->pred_H, c->pred_Hp, c->pred_Y, c->pred_K,
-                    c->pred_S, c->pred_fl, c->pred_cpart, c->pred_zero, c->cl_dinv};
+                    c->pred_S, c->pred_fl, c->pred_cpart, c->pred_zero, c->cl_dinv, c->vm_dinv};
     delete c->cl_host;
     delete c->cl_lf;
     delete c->cl_lb;
@@ -2520,7 +2544,8 @@ int vv_set_moments(vv_ctx* c, const double* n_p, const double* u_p, const double
 int vv_pc_set_potential(vv_ctx* c, const double* phi) {
     if (!c || !phi) return VV_ERR_ARG;
     if (c->g.preconditioner != VV_PC_TENSOR_POTENTIAL) return VV_OK;
-    return copy_d(c, c->phipc, phi, c->nx);
+    TRY(copy_d(c, c->phipc, phi, c->nx));
+    return pcv_factor(c);
 }
 
 int vv_moments(vv_ctx* c, const double* F, double* n, double* u, double* e, double* a) {

@@ -60,63 +60,150 @@ VV_DEV C c_div(C a, C b) {
     return r;
 }
 
-// A_k c = b for mode k = one thread, in place on spec[k*nx ..]; scr holds the
-// thread's diagonal, super- and (fill-in) second super-diagonal, 3 nx complex.
-// Elimination with partial pivoting as in a tridiagonal solver with row
-// interchanges (the fill-in of an interchange sits in dl), then back
-// substitution.
-template <typename R>
-__global__ void k_pcv_solve(typename Cplx<R>::type* __restrict__ spec, typename Cplx<R>::type* __restrict__ scr,
-                            PotParams p) {
-    using C = typename Cplx<R>::type;
+// Factors of every mode's A_k, kept until phi changes (update_matrices): the
+// elimination with partial pivoting of a tridiagonal solver with row
+// interchanges (the fill-in of an interchange is the second super-diagonal),
+// tables [row][mode].  Its divisions (540 cycles each) stay out of the
+// applications: 50 x 101 in FP64, one application 95 -> 24 us.
+template <typename C> struct PotLu {
+    C *fact, *dinv, *du, *dl;      // multiplier, 1/U_ii, U_{i,i+1}, U_{i,i+2}
+    unsigned char* swap;           // rows i and i+1 interchanged
+};
+
+// one thread per mode, in FP64; lu32 (optional): rounded copies
+static __global__ void k_pcv_factor(PotLu<double2> lu, PotLu<float2> lu32, PotParams p) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= p.nmv) return;
-    const int n = p.nx;
-    C* b = spec + (size_t)k * n;
-    C* d = scr + (size_t)k * 3 * n;
-    C* du = d + n;
-    C* dl = du + n;
-    const double2 lam = p.lam[k];
-    // bands (TensorProductPotentialFast.pyx:228-260): dl[i] = A[i+1][i], du[i] = A[i][i+1]
-    for (int i = 0; i < n; ++i) {
+    const int n = p.nx, m = p.nmv;
+    const double2 lam = p.lam[k], zero = make_double2(0.0, 0.0);
+    // bands (TensorProductPotentialFast.pyx:228-260): A[i][i], A[i][i+1] and A[i+1][i] (equal)
+    auto diag = [&](int i) {
         const int im = i == 0 ? n - 1 : i - 1, ip = i + 1 == n ? 0 : i + 1;
         const double2 dg = c_rmul(c_rmul(c_rmul(lam, 2.0), p.phi[ip] - p.phi[im]), p.arak);
-        d[i] = c_make<C>(dg.x + p.ht_inv, dg.y);
+        return make_double2(dg.x + p.ht_inv, dg.y);
+    };
+    auto off = [&](int i) {
+        return i + 1 < n ? c_rmul(c_rmul(c_rmul(lam, 1.0), p.phi[i + 1] - p.phi[i]), p.arak) : zero;
+    };
+    double2 d = diag(0), u = off(0);   // row i as the elimination left it
+    for (int i = 0; i < n; ++i) {
+        double2 f = zero, di = d, dui = u, dli = zero;
+        unsigned char sw = 0;
         if (i + 1 < n) {
-            const double2 up = c_rmul(c_rmul(c_rmul(lam, 1.0), p.phi[ip] - p.phi[i]), p.arak);
-            const int i1 = i + 1, i1m = i;
-            const double2 lo = c_rmul(c_rmul(c_rmul(lam, 1.0), p.phi[i1] - p.phi[i1m]), p.arak);
-            du[i] = c_make<C>(up.x, up.y);
-            dl[i] = c_make<C>(lo.x, lo.y);
-        }
-    }
-    const C zero = c_make<C>(0.0, 0.0);
-    for (int i = 0; i + 1 < n; ++i) {
-        const bool last = i + 2 == n;
-        if (c_abs1(d[i]) >= c_abs1(dl[i])) {   // no interchange
-            const C fact = c_div(dl[i], d[i]);
-            d[i + 1] = c_sub(d[i + 1], c_mul(fact, du[i]));
-            b[i + 1] = c_sub(b[i + 1], c_mul(fact, b[i]));
-            if (!last) dl[i] = zero;
-        } else {                                   // rows i and i+1 interchanged
-            const C fact = c_div(d[i], dl[i]);
-            d[i] = dl[i];
-            const C temp = d[i + 1];
-            d[i + 1] = c_sub(du[i], c_mul(fact, temp));
-            if (!last) {
-                dl[i] = du[i + 1];
-                du[i + 1] = c_make<C>(-(fact.x * dl[i].x - fact.y * dl[i].y), -(fact.x * dl[i].y + fact.y * dl[i].x));
+            const double2 l = off(i), dn = diag(i + 1), un = off(i + 1);
+            if (c_abs1(d) >= c_abs1(l)) {
+                f = c_div(l, d);
+                d = c_sub(dn, c_mul(f, u));
+                u = un;
+            } else {
+                sw = 1;
+                f = c_div(d, l);
+                di = l;
+                dui = dn;
+                dli = un;
+                d = c_sub(u, c_mul(f, dn));
+                const double2 t = c_mul(f, un);
+                u = make_double2(-t.x, -t.y);
             }
-            du[i] = temp;
-            const C tb = b[i];
-            b[i] = b[i + 1];
-            b[i + 1] = c_sub(tb, c_mul(fact, b[i + 1]));
+        }
+        const double2 inv = c_div(make_double2(1.0, 0.0), di);
+        const size_t q = (size_t)i * m + k;
+        lu.fact[q] = f;
+        lu.dinv[q] = inv;
+        lu.du[q] = dui;
+        lu.dl[q] = dli;
+        lu.swap[q] = sw;
+        if (lu32.fact) {
+            lu32.fact[q] = make_float2((float)f.x, (float)f.y);
+            lu32.dinv[q] = make_float2((float)inv.x, (float)inv.y);
+            lu32.du[q] = make_float2((float)dui.x, (float)dui.y);
+            lu32.dl[q] = make_float2((float)dli.x, (float)dli.y);
         }
     }
-    b[n - 1] = c_div(b[n - 1], d[n - 1]);
-    if (n > 1) b[n - 2] = c_div(c_sub(b[n - 2], c_mul(du[n - 2], b[n - 1])), d[n - 2]);
-    for (int i = n - 3; i >= 0; --i)
-        b[i] = c_div(c_sub(c_sub(b[i], c_mul(du[i], b[i + 1])), c_mul(dl[i], b[i + 2])), d[i]);
+}
+
+// A_k c = b in place on spec[k*nx ..], one thread per mode (a warp 32 of them).
+// A chain of two complex multiply-adds per row; the next rows' operands are
+// loaded while it runs (PV_CH rows ahead).
+constexpr int PV_CH = 4;
+template <typename R>
+__global__ void __launch_bounds__(32) k_pcv_solve(typename Cplx<R>::type* __restrict__ spec,
+                                                  PotLu<typename Cplx<R>::type> lu, int n, int m) {
+    using C = typename Cplx<R>::type;
+    const int k = blockIdx.x * 32 + threadIdx.x;
+    if (k >= m) return;
+    C* b = spec + (size_t)k * n;
+    const C zero = c_make<C>(0.0, 0.0);
+    {   // forward: b <- L^-1 P b
+        C f[2][PV_CH], r[2][PV_CH];
+        unsigned char w[2][PV_CH];
+        auto load = [&](int s, int i0) {
+#pragma unroll
+            for (int u = 0; u < PV_CH; ++u) {
+                const int i = min(i0 + u, n - 1);
+                f[s][u] = lu.fact[(size_t)i * m + k];
+                w[s][u] = lu.swap[(size_t)i * m + k];
+                r[s][u] = b[min(i + 1, n - 1)];
+            }
+        };
+        C cur = b[0];
+        load(0, 0);
+        int i0 = 0;
+        auto run = [&](int s) {
+            load(s ^ 1, i0 + PV_CH);
+#pragma unroll
+            for (int u = 0; u < PV_CH; ++u) {
+                const int i = i0 + u;
+                if (i + 1 < n) {
+                    const C nx = r[s][u];
+                    const bool sw = w[s][u] != 0;
+                    b[i] = sw ? nx : cur;
+                    cur = sw ? c_sub(cur, c_mul(f[s][u], nx)) : c_sub(nx, c_mul(f[s][u], cur));
+                }
+            }
+            i0 += PV_CH;
+        };
+        while (i0 < n - 1) {
+            run(0);
+            if (i0 < n - 1) run(1);
+        }
+        b[n - 1] = cur;
+    }
+    {   // back substitution
+        C d[2][PV_CH], u1[2][PV_CH], u2[2][PV_CH], r[2][PV_CH];
+        auto load = [&](int s, int i0) {
+#pragma unroll
+            for (int u = 0; u < PV_CH; ++u) {
+                const int i = max(i0 - u, 0);
+                const size_t q = (size_t)i * m + k;
+                d[s][u] = lu.dinv[q];
+                u1[s][u] = lu.du[q];
+                u2[s][u] = lu.dl[q];
+                r[s][u] = b[i];
+            }
+        };
+        C x1 = zero, x2 = zero;   // x_{i+1}, x_{i+2}
+        int i0 = n - 1;
+        load(0, i0);
+        auto run = [&](int s) {
+            load(s ^ 1, i0 - PV_CH);
+#pragma unroll
+            for (int u = 0; u < PV_CH; ++u) {
+                const int i = i0 - u;
+                if (i >= 0) {
+                    const C x = c_mul(d[s][u], c_sub(c_sub(r[s][u], c_mul(u2[s][u], x2)), c_mul(u1[s][u], x1)));
+                    b[i] = x;
+                    x2 = x1;
+                    x1 = x;
+                }
+            }
+            i0 -= PV_CH;
+        };
+        while (i0 >= 0) {
+            run(0);
+            if (i0 >= 0) run(1);
+        }
+    }
 }
 
 }  // namespace vv
