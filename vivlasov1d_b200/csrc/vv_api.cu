@@ -509,8 +509,12 @@ size_t fft_smem(int kind, int M, int R, size_t csz, bool inverse) {
 bool four_step_ok(int M) { return M >= 32 && M <= 512; }
 
 // shared memory of the direct-DFT kernels (any nx)
-size_t rdft_smem(int nx, size_t csz) { return (size_t)nx * csz + (size_t)vv::DFT_ROWS * nx * (csz / 2); }
-size_t irdft_smem(int nx, size_t csz) { return (size_t)nx * csz + (size_t)vv::DFT_ROWS * (nx / 2 + 1) * csz; }
+size_t rdft_smem(int nx, size_t csz) {
+    const size_t nm = nx / 2 + 1, nT = (nm + 31) / 32;
+    const size_t red = nT >= (size_t)vv::DFT_WARPS ? 0 : (size_t)vv::DFT_WARPS * vv::DFT_ROWS * 32;
+    return ((size_t)nx + vv::DFT_ROWS * nm + red) * csz;
+}
+size_t irdft_smem(int nx, size_t csz) { return rdft_smem(nx, csz); }
 
 template <typename TI, typename R>
 int launch_rfft(vv_ctx* c, const TI* X, typename Cplx<R>::type* spec, const vv::PcParams& p, unsigned rows) {

@@ -418,45 +418,113 @@ __global__ void k_irfft4(const typename Cplx<R>::type* __restrict__ spec, TO* __
 // configurations).  O(nx^2) per row from the nx-entry twiddle table;
 // numpy's rfft / irfft conventions (irfft ignores the imaginary parts of
 // X_0 and, for even nx, X_{nx/2}).  DFT_ROWS rows per CTA.
+// A warp takes 32 modes (samples) of the block's rows, so that a twiddle gathered
+// from shared memory serves DFT_ROWS products; x_n and x_{nx-n} share it too (their
+// sum and difference are staged).  With fewer than eight tiles of modes the
+// sum over n is split over the warps.  201 x 401 in FP64: forward 13.6 -> 5.5 us,
+// inverse 15.8 -> 6.0 us.
 // ---------------------------------------------------------------------------
-constexpr int DFT_ROWS = 4, DFT_THREADS = 256;
+constexpr int DFT_ROWS = 4, DFT_THREADS = 256, DFT_WARPS = DFT_THREADS / 32;
+
+// the warp's tile and share of the sum: parts warps per tile
+struct DftSplit {
+    int nT, parts, tile, part, step;
+    VV_DEV explicit DftSplit(int nm) {
+        const int w = threadIdx.x >> 5;
+        nT = (nm + 31) >> 5;
+        parts = nT >= DFT_WARPS ? 1 : DFT_WARPS / nT;
+        tile = nT >= DFT_WARPS ? w : w % nT;
+        part = nT >= DFT_WARPS ? 0 : w / nT;
+        step = nT >= DFT_WARPS ? DFT_WARPS : nT;   // one tile per warp, or a loop over tiles
+    }
+};
+// sum of the parts' (a, b) of every row; valid in part 0
+template <typename C>
+VV_DEV void dft_join(C (&v)[DFT_ROWS], const DftSplit& s, C* red) {
+    const int lane = threadIdx.x & 31;
+    if (s.parts == 1) return;
+    if (s.part > 0 && s.part < s.parts) {
+#pragma unroll
+        for (int r = 0; r < DFT_ROWS; ++r) red[(((s.part - 1) * s.nT + s.tile) * DFT_ROWS + r) * 32 + lane] = v[r];
+    }
+    __syncthreads();
+    if (s.part == 0) {
+        for (int q = 1; q < s.parts; ++q)
+#pragma unroll
+            for (int r = 0; r < DFT_ROWS; ++r)
+                v[r] = c_add(v[r], red[(((q - 1) * s.nT + s.tile) * DFT_ROWS + r) * 32 + lane]);
+    }
+}
 
 // X_k = sum_n x_n W^{nk}, k = 0..nx/2, written mode-major spec[k*nv + j].
-// dynamic smem: nx twiddles (complex R) + DFT_ROWS x nx (R)
+// dynamic smem: nx twiddles, DFT_ROWS x (nx/2 + 1) pairs, the parts' sums (complex R)
 template <typename TI, typename R>
 __global__ void __launch_bounds__(DFT_THREADS)
 k_rdft_rows(const TI* __restrict__ X, typename Cplx<R>::type* __restrict__ spec, PcParams p) {
     using C = typename Cplx<R>::type;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int N = p.nx, nm = N / 2 + 1;
+    const int N = p.nx, nm = N / 2 + 1, half = (N - 1) / 2;
     C* stw = reinterpret_cast<C*>(smem_raw);
-    R* xs = reinterpret_cast<R*>(stw + N);
+    C* xs = stw + N;             // row r: (x_0, x_{N/2} or 0), then (x_n + x_{N-n}, x_n - x_{N-n})
+    C* red = xs + DFT_ROWS * nm;
     const C* tw = reinterpret_cast<const C*>(p.tw);
     for (int k = threadIdx.x; k < N; k += blockDim.x) stw[k] = tw[k];
     const int j0 = blockIdx.x * DFT_ROWS;
-    for (int i = threadIdx.x; i < DFT_ROWS * N; i += blockDim.x) {
-        const int r = i / N, n = i - r * N, j = j0 + r;
-        xs[i] = (j < p.nv) ? (R)X[(size_t)j * N + n] : (R)0;
+    for (int i = threadIdx.x; i < DFT_ROWS * (half + 1); i += blockDim.x) {
+        const int r = i / (half + 1), n = i - r * (half + 1), j = j0 + r;
+        C v;
+        v.x = v.y = R(0);
+        if (j < p.nv) {
+            const TI* row = X + (size_t)j * N;
+            if (n == 0) {
+                v.x = (R)row[0];
+                if (!(N & 1)) v.y = (R)row[N / 2];
+            } else {
+                const R a = (R)row[n], b = (R)row[N - n];
+                v.x = a + b;
+                v.y = a - b;
+            }
+        }
+        xs[r * nm + n] = v;
     }
     __syncthreads();
-    for (int u = threadIdx.x; u < nm * DFT_ROWS; u += blockDim.x) {
-        const int k = u / DFT_ROWS, r = u - k * DFT_ROWS, j = j0 + r;
-        const R* xr = xs + r * N;
-        R re = 0, im = 0;
-        int idx = 0;
-        for (int n = 0; n < N; ++n) {
-            const C w = stw[idx];
-            re += xr[n] * w.x;
-            im += xr[n] * w.y;
-            idx += k;
-            if (idx >= N) idx -= N;
+    const DftSplit s(nm);
+    for (int tile = s.tile; tile < s.nT; tile += s.step) {
+        const int k = tile * 32 + (threadIdx.x & 31), kk = k < nm ? k : 0;
+        C v[DFT_ROWS];
+#pragma unroll
+        for (int r = 0; r < DFT_ROWS; ++r) {
+            const C e = xs[r * nm];
+            v[r].x = s.part == 0 ? e.x + ((kk & 1) ? -e.y : e.y) : R(0);
+            v[r].y = R(0);
         }
-        if (j < p.nv) spec[(size_t)k * p.nv + j] = c_make<C>((double)re, (double)im);
+        if (s.part < s.parts) {
+            const int na = 1 + s.part * half / s.parts, nb = 1 + (s.part + 1) * half / s.parts;
+            int idx = (int)((long long)kk * na % N);
+#pragma unroll 2
+            for (int n = na; n < nb; ++n) {
+                const C w = stw[idx];
+#pragma unroll
+                for (int r = 0; r < DFT_ROWS; ++r) {
+                    const C x = xs[r * nm + n];
+                    v[r].x += x.x * w.x;
+                    v[r].y += x.y * w.y;
+                }
+                idx += kk;
+                if (idx >= N) idx -= N;
+            }
+        }
+        dft_join(v, s, red);
+        if (s.part == 0 && k < nm) {
+#pragma unroll
+            for (int r = 0; r < DFT_ROWS; ++r)
+                if (j0 + r < p.nv) spec[(size_t)k * p.nv + j0 + r] = v[r];
+        }
     }
 }
 
-// x_n = (1/nx) [Re X_0 + 2 sum_{k=1}^{(nx-1)/2} Re(X_k W^{-nk}) + (nx even) Re X_{nx/2} (-1)^n]
-// dynamic smem: nx twiddles + DFT_ROWS x (nx/2 + 1) complex
+// x_n = (1/nx) [Re X_0 + 2 sum_{k=1}^{(nx-1)/2} Re(X_k W^{-nk}) + (nx even) Re X_{nx/2} (-1)^n],
+// a lane the samples n and nx - n.  dynamic smem as k_rdft_rows
 template <typename R, typename TO>
 __global__ void __launch_bounds__(DFT_THREADS)
 k_irdft_rows(const typename Cplx<R>::type* __restrict__ spec, TO* __restrict__ Y, PcParams p) {
@@ -466,6 +534,7 @@ k_irdft_rows(const typename Cplx<R>::type* __restrict__ spec, TO* __restrict__ Y
     const int N = p.nx, nm = N / 2 + 1, K = (N - 1) / 2;
     C* stw = reinterpret_cast<C*>(smem_raw);
     C* xs = stw + N;
+    C* red = xs + DFT_ROWS * nm;
     const C* tw = reinterpret_cast<const C*>(p.tw);
     for (int k = threadIdx.x; k < N; k += blockDim.x) stw[k] = tw[k];
     const int j0 = blockIdx.x * DFT_ROWS;
@@ -475,19 +544,41 @@ k_irdft_rows(const typename Cplx<R>::type* __restrict__ spec, TO* __restrict__ Y
     }
     __syncthreads();
     const R inv = (R)(1.0 / (double)N);
-    for (int u = threadIdx.x; u < DFT_ROWS * N; u += blockDim.x) {
-        const int r = u / N, n = u - r * N, j = j0 + r;
-        const C* xr = xs + r * nm;
-        R s = xr[0].x;
-        int idx = 0;
-        for (int k = 1; k <= K; ++k) {
-            idx += n;
-            if (idx >= N) idx -= N;
-            const C w = stw[idx];   // W^{nk} = (cos, -sin): Re(X e^{+i theta}) = X.x w.x + X.y w.y
-            s += (R)2 * (xr[k].x * w.x + xr[k].y * w.y);
+    const DftSplit s(nm);
+    for (int tile = s.tile; tile < s.nT; tile += s.step) {
+        const int n = tile * 32 + (threadIdx.x & 31), nn = n < nm ? n : 0;
+        C v[DFT_ROWS];   // sum of Re X cos, of -Im X sin
+#pragma unroll
+        for (int r = 0; r < DFT_ROWS; ++r) v[r].x = v[r].y = R(0);
+        if (s.part < s.parts) {
+            const int ka = 1 + s.part * K / s.parts, kb = 1 + (s.part + 1) * K / s.parts;
+            int idx = (int)((long long)nn * ka % N);
+#pragma unroll 2
+            for (int k = ka; k < kb; ++k) {
+                const C w = stw[idx];   // W^{nk} = (cos, -sin): Re(X e^{+i theta}) = X.x w.x + X.y w.y
+#pragma unroll
+                for (int r = 0; r < DFT_ROWS; ++r) {
+                    const C x = xs[r * nm + k];
+                    v[r].x += x.x * w.x;
+                    v[r].y += x.y * w.y;
+                }
+                idx += nn;
+                if (idx >= N) idx -= N;
+            }
         }
-        if (!(N & 1)) s += (n & 1) ? -xr[N / 2].x : xr[N / 2].x;
-        if (j < p.nv) Y[(size_t)j * N + n] = (TO)(s * inv);
+        dft_join(v, s, red);
+        if (s.part == 0 && n < nm) {
+#pragma unroll
+            for (int r = 0; r < DFT_ROWS; ++r)
+                if (j0 + r < p.nv) {
+                    const C* xr = xs + r * nm;
+                    R e = xr[0].x;
+                    if (!(N & 1)) e += (n & 1) ? -xr[N / 2].x : xr[N / 2].x;
+                    TO* row = Y + (size_t)(j0 + r) * N;
+                    row[n] = (TO)((e + (R)2 * (v[r].x + v[r].y)) * inv);
+                    if (n > 0 && 2 * n != N) row[N - n] = (TO)((e + (R)2 * (v[r].x - v[r].y)) * inv);
+                }
+        }
     }
 }
 
