@@ -522,7 +522,7 @@ int launch_rfft(vv_ctx* c, const TI* X, typename Cplx<R>::type* spec, const vv::
     const int M = c->M;
     if (c->fft_kind == 2 || !c->pow2) {
         const unsigned g = (unsigned)((c->nv + vv::DFT_ROWS - 1) / vv::DFT_ROWS);
-        vv::k_rdft_rows<TI, R><<<g, vv::DFT_THREADS, rdft_smem(c->nx, csz), c->st>>>(X, spec, p);
+        vv::k_rdft_rows<TI, R><<<g, vv::DFT_THREADS, rdft_smem(c->nx, csz), c->st>>>(X, spec, p, 0);
     } else if (c->fft_kind == 1 && four_step_ok(M)) {
         const size_t sm = fft_smem(1, M, c->pcR, csz, false);
         switch (M / 32) {
@@ -545,7 +545,7 @@ int launch_irfft(vv_ctx* c, const typename Cplx<R>::type* spec, TO* Y, const vv:
     const int M = c->M;
     if (c->fft_kind == 2 || !c->pow2) {
         const unsigned g = (unsigned)((c->nv + vv::DFT_ROWS - 1) / vv::DFT_ROWS);
-        vv::k_irdft_rows<R, TO><<<g, vv::DFT_THREADS, irdft_smem(c->nx, csz), c->st>>>(spec, Y, p);
+        vv::k_irdft_rows<R, TO><<<g, vv::DFT_THREADS, irdft_smem(c->nx, csz), c->st>>>(spec, Y, p, 0);
     } else if (c->fft_kind == 1 && four_step_ok(M)) {
         const size_t sm = fft_smem(1, M, c->pcR, csz, true);
         switch (M / 32) {
@@ -594,6 +594,9 @@ void smem_attributes(int optin, int& lowest, cudaError_t& e) {
     set((const void*)vv::k_rdft_rows<double, R>);
     set((const void*)vv::k_rdft_rows<float, R>);
     set((const void*)vv::k_irdft_rows<R, R>);
+    set((const void*)vv::k_rdft_rows<double, R, true>);
+    set((const void*)vv::k_rdft_rows<float, R, true>);
+    set((const void*)vv::k_irdft_rows<R, R, true>);
     set((const void*)vv::k_tridiag_warp_staged<R>);
     set((const void*)vv::k_b_tridiag_w<R>);
     set((const void*)vv::k_b_rfftj<double, R>);
@@ -870,8 +873,9 @@ int pcv_factor(vv_ctx* c) {
 }
 
 // The potential preconditioner: the v transforms as row transforms of the
-// transposed field (radix-2 FFT for a power-of-two nv, else the direct DFT),
-// the x-tridiagonal systems per v mode from their factors
+// transposed field (radix-2 FFT for a power-of-two nv) or on the field's
+// columns in place (the direct DFT, whose rows are staged in shared memory
+// anyway: no transposes), the x-tridiagonal systems per v mode from their factors
 template <typename TI, typename R, typename TO>
 int pcv_apply_t(vv_ctx* c, const TI* X, TO* Y, const int* yidx = nullptr, int yoff = 0) {
     constexpr bool D = std::is_same<R, double>::value;
@@ -880,8 +884,11 @@ int pcv_apply_t(vv_ctx* c, const TI* X, TO* Y, const int* yidx = nullptr, int yo
     R* xt = D ? reinterpret_cast<R*>(c->pv_xt) : reinterpret_cast<R*>(c->pv_xt32);
     C2* spec = D ? reinterpret_cast<C2*>(c->pv_spec) : reinterpret_cast<C2*>(c->pv_spec32);
     const dim3 tb(32, 8);
-    vv::k_transpose<TI, R><<<dim3((nx + 31) / 32, (nv + 31) / 32), tb, 0, c->st>>>(X, xt, nv, nx, nullptr, 0, 0);
-    CKL(c);
+    const bool fft = is_pow2(nv);
+    if (fft) {
+        vv::k_transpose<TI, R><<<dim3((nx + 31) / 32, (nv + 31) / 32), tb, 0, c->st>>>(X, xt, nv, nx, nullptr, 0, 0);
+        CKL(c);
+    }
     vv::PcParams p;
     p.nx = nv;   // rows of length nv ...
     p.nv = nx;   // ... one per x point
@@ -893,17 +900,30 @@ int pcv_apply_t(vv_ctx* c, const TI* X, TO* Y, const int* yidx = nullptr, int yo
     p.yoff = 0;
     p.ystride = 0;
     const size_t csz = sizeof(C2);
-    const bool fft = is_pow2(nv);
     const unsigned gr = (unsigned)((nx + c->pvR - 1) / c->pvR), gd = (unsigned)((nx + vv::DFT_ROWS - 1) / vv::DFT_ROWS);
     if (fft) vv::k_rfft_rows<R, R><<<gr, 32 * c->pvR, fft_smem(0, nv / 2, c->pvR, csz, false), c->st>>>(xt, spec, p);
-    else vv::k_rdft_rows<R, R><<<gd, vv::DFT_THREADS, rdft_smem(nv, csz), c->st>>>(xt, spec, p);
+    else vv::k_rdft_rows<TI, R, true><<<gd, vv::DFT_THREADS, rdft_smem(nv, csz), c->st>>>(X, spec, p, nx);   // rows = the field's columns
     CKL(c);
-    const unsigned gm = (unsigned)((c->nmv + 31) / 32);
-    if constexpr (D) vv::k_pcv_solve<double><<<gm, 32, 0, c->st>>>(spec, c->pv_lu, nx, c->nmv);
-    else vv::k_pcv_solve<float><<<gm, 32, 0, c->st>>>(spec, c->pv_lu32, nx, c->nmv);
+    const vv::PotLu<C2>& lu = [&]() -> const vv::PotLu<C2>& {
+        if constexpr (D) return c->pv_lu;
+        else return c->pv_lu32;
+    }();
+    int mb = 8;   // modes of a block: as many as the shared memory holds
+    while (mb > 0 && vv::pcv_smem(csz, nx, mb) > vv::PV_SMEM) mb /= 2;
+    if (mb > 0)
+        vv::k_pcv_solve_sm<R><<<(unsigned)((c->nmv + mb - 1) / mb), vv::PV_THREADS, vv::pcv_smem(csz, nx, mb), c->st>>>(
+            spec, lu, nx, c->nmv, mb);
+    else vv::k_pcv_solve<R><<<(unsigned)((c->nmv + 31) / 32), 32, 0, c->st>>>(spec, lu, nx, c->nmv);
     CKL(c);
     if (fft) vv::k_irfft_rows<R, R><<<gr, 32 * c->pvR, fft_smem(0, nv / 2, c->pvR, csz, true), c->st>>>(spec, xt, p);
-    else vv::k_irdft_rows<R, R><<<gd, vv::DFT_THREADS, irdft_smem(nv, csz), c->st>>>(spec, xt, p);
+    else {
+        p.yidx = yidx;
+        p.yoff = yoff;
+        p.ystride = yidx ? c->ncell : 0;
+        vv::k_irdft_rows<R, TO, true><<<gd, vv::DFT_THREADS, irdft_smem(nv, csz), c->st>>>(spec, Y, p, nx);
+        CKL(c);
+        return VV_OK;
+    }
     CKL(c);
     vv::k_transpose<R, TO><<<dim3((nv + 31) / 32, (nx + 31) / 32), tb, 0, c->st>>>(xt, Y, nx, nv, yidx, yoff,
                                                                                    yidx ? c->ncell : 0);

@@ -421,8 +421,8 @@ __global__ void k_irfft4(const typename Cplx<R>::type* __restrict__ spec, TO* __
 // A warp takes 32 modes (samples) of the block's rows, so that a twiddle gathered
 // from shared memory serves DFT_ROWS products; x_n and x_{nx-n} share it too (their
 // sum and difference are staged).  With fewer than eight tiles of modes the
-// sum over n is split over the warps.  201 x 401 in FP64: forward 13.6 -> 5.5 us,
-// inverse 15.8 -> 6.0 us.
+// sum over n is split over the warps.  201 x 401 in FP64: forward 8.5 us,
+// inverse 9.2 us, the function call that holds them 49 -> 28.7 us.
 // ---------------------------------------------------------------------------
 constexpr int DFT_ROWS = 4, DFT_THREADS = 256, DFT_WARPS = DFT_THREADS / 32;
 
@@ -458,9 +458,12 @@ VV_DEV void dft_join(C (&v)[DFT_ROWS], const DftSplit& s, C* red) {
 
 // X_k = sum_n x_n W^{nk}, k = 0..nx/2, written mode-major spec[k*nv + j].
 // dynamic smem: nx twiddles, DFT_ROWS x (nx/2 + 1) pairs, the parts' sums (complex R)
-template <typename TI, typename R>
+// COLS: the rows transformed are the columns of a field `cols` wide (an argument
+// of these kernels alone: a wider PcParams changes how the other kernels'
+// complex products are rounded)
+template <typename TI, typename R, bool COLS = false>
 __global__ void __launch_bounds__(DFT_THREADS)
-k_rdft_rows(const TI* __restrict__ X, typename Cplx<R>::type* __restrict__ spec, PcParams p) {
+k_rdft_rows(const TI* __restrict__ X, typename Cplx<R>::type* __restrict__ spec, PcParams p, int cols) {
     using C = typename Cplx<R>::type;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int N = p.nx, nm = N / 2 + 1, half = (N - 1) / 2;
@@ -471,16 +474,18 @@ k_rdft_rows(const TI* __restrict__ X, typename Cplx<R>::type* __restrict__ spec,
     for (int k = threadIdx.x; k < N; k += blockDim.x) stw[k] = tw[k];
     const int j0 = blockIdx.x * DFT_ROWS;
     for (int i = threadIdx.x; i < DFT_ROWS * (half + 1); i += blockDim.x) {
-        const int r = i / (half + 1), n = i - r * (half + 1), j = j0 + r;
+        // sample n of row j at j N + n, or at n cols + j
+        const int r = COLS ? i % DFT_ROWS : i / (half + 1), n = COLS ? i / DFT_ROWS : i - r * (half + 1), j = j0 + r;
         C v;
         v.x = v.y = R(0);
         if (j < p.nv) {
-            const TI* row = X + (size_t)j * N;
+            const TI* row = X + (COLS ? (size_t)j : (size_t)j * N);
+            const size_t es = COLS ? (size_t)cols : 1;
             if (n == 0) {
                 v.x = (R)row[0];
-                if (!(N & 1)) v.y = (R)row[N / 2];
+                if (!(N & 1)) v.y = (R)row[(N / 2) * es];
             } else {
-                const R a = (R)row[n], b = (R)row[N - n];
+                const R a = (R)row[n * es], b = (R)row[(N - n) * es];
                 v.x = a + b;
                 v.y = a - b;
             }
@@ -525,9 +530,9 @@ k_rdft_rows(const TI* __restrict__ X, typename Cplx<R>::type* __restrict__ spec,
 
 // x_n = (1/nx) [Re X_0 + 2 sum_{k=1}^{(nx-1)/2} Re(X_k W^{-nk}) + (nx even) Re X_{nx/2} (-1)^n],
 // a lane the samples n and nx - n.  dynamic smem as k_rdft_rows
-template <typename R, typename TO>
+template <typename R, typename TO, bool COLS = false>
 __global__ void __launch_bounds__(DFT_THREADS)
-k_irdft_rows(const typename Cplx<R>::type* __restrict__ spec, TO* __restrict__ Y, PcParams p) {
+k_irdft_rows(const typename Cplx<R>::type* __restrict__ spec, TO* __restrict__ Y, PcParams p, int cols) {
     using C = typename Cplx<R>::type;
     if (p.yidx) Y += (size_t)(*p.yidx + p.yoff) * p.ystride;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -574,9 +579,10 @@ k_irdft_rows(const typename Cplx<R>::type* __restrict__ spec, TO* __restrict__ Y
                     const C* xr = xs + r * nm;
                     R e = xr[0].x;
                     if (!(N & 1)) e += (n & 1) ? -xr[N / 2].x : xr[N / 2].x;
-                    TO* row = Y + (size_t)(j0 + r) * N;
-                    row[n] = (TO)((e + (R)2 * (v[r].x + v[r].y)) * inv);
-                    if (n > 0 && 2 * n != N) row[N - n] = (TO)((e + (R)2 * (v[r].x - v[r].y)) * inv);
+                    TO* row = Y + (COLS ? (size_t)(j0 + r) : (size_t)(j0 + r) * N);
+                    const size_t es = COLS ? (size_t)cols : 1;
+                    row[n * es] = (TO)((e + (R)2 * (v[r].x + v[r].y)) * inv);
+                    if (n > 0 && 2 * n != N) row[(N - n) * es] = (TO)((e + (R)2 * (v[r].x - v[r].y)) * inv);
                 }
         }
     }

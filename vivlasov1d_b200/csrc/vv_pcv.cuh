@@ -15,7 +15,7 @@
 // The v transforms run as the x-row kernels on the transposed field (rows of
 // length nv); A_k is solved by Gaussian elimination with partial pivoting
 // (the pivot rule of LAPACK's band LU: swap when |sub|_1 > |diag|_1), one
-// thread per mode, rebuilt at every application from phi.
+// thread per mode; the factors are made once per phi.
 #pragma once
 #include "vv_common.cuh"
 
@@ -64,7 +64,7 @@ VV_DEV C c_div(C a, C b) {
 // elimination with partial pivoting of a tridiagonal solver with row
 // interchanges (the fill-in of an interchange is the second super-diagonal),
 // tables [row][mode].  Its divisions (540 cycles each) stay out of the
-// applications: 50 x 101 in FP64, one application 95 -> 24 us.
+// applications.
 template <typename C> struct PotLu {
     C *fact, *dinv, *du, *dl;      // multiplier, 1/U_ii, U_{i,i+1}, U_{i,i+2}
     unsigned char* swap;           // rows i and i+1 interchanged
@@ -122,17 +122,13 @@ static __global__ void k_pcv_factor(PotLu<double2> lu, PotLu<float2> lu32, PotPa
     }
 }
 
-// A_k c = b in place on spec[k*nx ..], one thread per mode (a warp 32 of them).
-// A chain of two complex multiply-adds per row; the next rows' operands are
-// loaded while it runs (PV_CH rows ahead).
+// One mode's elimination and back substitution, row i of b at b + i bs, of the
+// factors at i m.  A chain of two complex multiply-adds per row; the next rows'
+// operands are loaded while it runs (PV_CH rows ahead).
 constexpr int PV_CH = 4;
-template <typename R>
-__global__ void __launch_bounds__(32) k_pcv_solve(typename Cplx<R>::type* __restrict__ spec,
-                                                  PotLu<typename Cplx<R>::type> lu, int n, int m) {
-    using C = typename Cplx<R>::type;
-    const int k = blockIdx.x * 32 + threadIdx.x;
-    if (k >= m) return;
-    C* b = spec + (size_t)k * n;
+template <typename C>
+VV_DEV void pcv_chain(C* b, int bs, const C* fact, const C* dinv, const C* du, const C* dl, const unsigned char* swap,
+                      int n, int m) {
     const C zero = c_make<C>(0.0, 0.0);
     {   // forward: b <- L^-1 P b
         C f[2][PV_CH], r[2][PV_CH];
@@ -141,9 +137,9 @@ __global__ void __launch_bounds__(32) k_pcv_solve(typename Cplx<R>::type* __rest
 #pragma unroll
             for (int u = 0; u < PV_CH; ++u) {
                 const int i = min(i0 + u, n - 1);
-                f[s][u] = lu.fact[(size_t)i * m + k];
-                w[s][u] = lu.swap[(size_t)i * m + k];
-                r[s][u] = b[min(i + 1, n - 1)];
+                f[s][u] = fact[(size_t)i * m];
+                w[s][u] = swap[(size_t)i * m];
+                r[s][u] = b[(size_t)min(i + 1, n - 1) * bs];
             }
         };
         C cur = b[0];
@@ -157,7 +153,7 @@ __global__ void __launch_bounds__(32) k_pcv_solve(typename Cplx<R>::type* __rest
                 if (i + 1 < n) {
                     const C nx = r[s][u];
                     const bool sw = w[s][u] != 0;
-                    b[i] = sw ? nx : cur;
+                    b[(size_t)i * bs] = sw ? nx : cur;
                     cur = sw ? c_sub(cur, c_mul(f[s][u], nx)) : c_sub(nx, c_mul(f[s][u], cur));
                 }
             }
@@ -167,7 +163,7 @@ __global__ void __launch_bounds__(32) k_pcv_solve(typename Cplx<R>::type* __rest
             run(0);
             if (i0 < n - 1) run(1);
         }
-        b[n - 1] = cur;
+        b[(size_t)(n - 1) * bs] = cur;
     }
     {   // back substitution
         C d[2][PV_CH], u1[2][PV_CH], u2[2][PV_CH], r[2][PV_CH];
@@ -175,11 +171,11 @@ __global__ void __launch_bounds__(32) k_pcv_solve(typename Cplx<R>::type* __rest
 #pragma unroll
             for (int u = 0; u < PV_CH; ++u) {
                 const int i = max(i0 - u, 0);
-                const size_t q = (size_t)i * m + k;
-                d[s][u] = lu.dinv[q];
-                u1[s][u] = lu.du[q];
-                u2[s][u] = lu.dl[q];
-                r[s][u] = b[i];
+                const size_t q = (size_t)i * m;
+                d[s][u] = dinv[q];
+                u1[s][u] = du[q];
+                u2[s][u] = dl[q];
+                r[s][u] = b[(size_t)i * bs];
             }
         };
         C x1 = zero, x2 = zero;   // x_{i+1}, x_{i+2}
@@ -192,7 +188,7 @@ __global__ void __launch_bounds__(32) k_pcv_solve(typename Cplx<R>::type* __rest
                 const int i = i0 - u;
                 if (i >= 0) {
                     const C x = c_mul(d[s][u], c_sub(c_sub(r[s][u], c_mul(u2[s][u], x2)), c_mul(u1[s][u], x1)));
-                    b[i] = x;
+                    b[(size_t)i * bs] = x;
                     x2 = x1;
                     x1 = x;
                 }
@@ -203,6 +199,54 @@ __global__ void __launch_bounds__(32) k_pcv_solve(typename Cplx<R>::type* __rest
             run(0);
             if (i0 >= 0) run(1);
         }
+    }
+}
+
+// A_k c = b in place on spec[k*nx ..], one thread per mode (a warp 32 of them),
+// for systems too long for shared memory
+template <typename R>
+__global__ void __launch_bounds__(32) k_pcv_solve(typename Cplx<R>::type* __restrict__ spec,
+                                                  PotLu<typename Cplx<R>::type> lu, int n, int m) {
+    const int k = blockIdx.x * 32 + threadIdx.x;
+    if (k >= m) return;
+    pcv_chain(spec + (size_t)k * n, 1, lu.fact + k, lu.dinv + k, lu.du + k, lu.dl + k, lu.swap + k, n, m);
+}
+
+// The same with a block's `mb` modes whole in shared memory: there are only
+// nv/2 + 1 chains, so a chain that waits for L2 every PV_CH rows leaves the chip
+// idle; here all operands are in flight at once and the chain reads shared memory
+// (50 x 101 in FP64: 17.4 -> 11.8 us; staging tiles of 8 rows ahead of the chain,
+// a barrier per tile, took 36).
+constexpr int PV_THREADS = 128;
+constexpr size_t PV_SMEM = 48 * 1024;
+inline size_t pcv_smem(size_t csz, int n, int mb) { return (size_t)n * mb * (5 * csz + 1); }
+template <typename R>
+__global__ void __launch_bounds__(PV_THREADS) k_pcv_solve_sm(typename Cplx<R>::type* __restrict__ spec,
+                                                             PotLu<typename Cplx<R>::type> lu, int n, int m, int mb) {
+    using C = typename Cplx<R>::type;
+    extern __shared__ __align__(16) unsigned char pv_raw[];
+    const int e1 = n * mb, k0 = blockIdx.x * mb, on = min(mb, m - k0);
+    C* b = reinterpret_cast<C*>(pv_raw);
+    C *f = b + e1, *d = f + e1, *u1 = d + e1, *u2 = u1 + e1;
+    unsigned char* w = reinterpret_cast<unsigned char*>(u2 + e1);
+    for (int e = threadIdx.x; e < n * on; e += PV_THREADS) {
+        const int i = e / on, l = e - i * on, t = i * mb + l;
+        const size_t q = (size_t)i * m + k0 + l;
+        f[t] = lu.fact[q];
+        d[t] = lu.dinv[q];
+        u1[t] = lu.du[q];
+        u2[t] = lu.dl[q];
+        w[t] = lu.swap[q];
+        const int lb = e / n, ib = e - lb * n;   // a mode's rows are contiguous
+        b[ib * mb + lb] = spec[(size_t)k0 * n + e];
+    }
+    __syncthreads();
+    const int l = threadIdx.x;
+    if (l < on) pcv_chain(b + l, mb, f + l, d + l, u1 + l, u2 + l, w + l, n, mb);
+    __syncthreads();
+    for (int e = threadIdx.x; e < n * on; e += PV_THREADS) {
+        const int lb = e / n, ib = e - lb * n;
+        spec[(size_t)k0 * n + e] = b[ib * mb + lb];
     }
 }
 
