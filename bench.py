@@ -11,11 +11,11 @@ instance by one implicit time step.  Gcell-steps/s = sum(nx nv) * steps / s.
 
     python bench.py [--gpus N] [--steps K] [--warmup W] [--impl reference]
 
-value       : batched + mixed precision -- every kernel launched once for the
-              instance table, lockstep Picard/GMRES loops with per-instance
-              masks, one CUDA graph per step; FP32 GMRES basis, Jacobian and
+value       : batched + mixed precision -- every instance that fits runs its
+              step on its own thread-block cluster, the others as one lockstep
+              table in a CUDA graph; FP32 GMRES basis, Jacobian and
               preconditioner, FP64 residual, Picard loop, moments, Poisson and
-              invariants; one lockstep table.
+              invariants; one batch.
               Device time of K steps (CUDA events), state resident in HBM
               (the working set is far larger than L2).
 plain_fp64  : the same instances in FP64, each advanced by its own vv_step
@@ -211,7 +211,7 @@ def run_gpu(args, rank, world):
     mixed = W.sweep_runs(specs=specs, device=dev, precision="mixed", snes_atol=SNES_ATOL)
     plain = W.sweep_runs(specs=specs, device=dev, precision="fp64", snes_atol=SNES_ATOL)
     bfp64 = W.sweep_runs(specs=specs, device=dev, precision="fp64", snes_atol=SNES_ATOL)
-    # mixed: one lockstep table; batched FP64: the first warm-up step whole,
+    # mixed: one batch; batched FP64: the first warm-up step whole,
     # the later steps with the slowest eighth of the instances as a second
     # table beside the rest
     batch = Batch(mixed)
@@ -411,7 +411,7 @@ def main():
     config = {"workload": WORKLOAD, "instances": N_INSTANCES, "seed": 20261203, "precision": "mixed",
               "mixed_inner_rtol": 1e-2, "ksp_rtol": 1e-4, "snes_atol": SNES_ATOL, "dt": 0.1,
               "bracket": "arakawaj4", "preconditioner": "tensor_kinetic", "parallelism": "replicas x%d" % args.gpus,
-              "tables": "one lockstep table (batched FP64: the slowest eighth of the instances and the rest, "
+              "tables": "one batch, instances on thread-block clusters where they fit (batched FP64: the slowest eighth of the instances and the rest, "
                         "stepped concurrently on two streams)",
               "l2": "working set far larger than L2 (17.5 M cells x ~40 fields); no flush",
               "host": "the harness's setup objects frozen out of Python's cyclic GC before the timed steps"}
@@ -468,7 +468,7 @@ def main():
     achieved = mdot_bytes / res["mdot_s"] / 1e9
     tri_gbps = tri_bytes / res["tri_s"] / 1e9
     roofline = {"kernel": "multi-dot of the Gram-Schmidt step (k_b_gm_mdot_p, whole table at Arnoldi index %d; "
-                          "the largest share of the step's launch list)" % MDOT_IT,
+                          "the largest share of the lockstep table's launch list)" % MDOT_IT,
                 "bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                 "peak_kind": peak_kind, "traffic": profiled_traffic("batch_mdot_traffic.json"),
                 "algorithmic_bytes_per_launch": mdot_bytes, "avg_launch_us": res["mdot_s"] * 1e6,

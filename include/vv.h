@@ -336,21 +336,23 @@ int vv_predict(vv_ctx* ctx, const double* F, const double* h1h, const double* h2
  * and whether the prediction was kept. */
 int vv_initial_guess(vv_ctx* ctx, vv_state* st, double* prev, double* guess, int32_t* kept);
 
-/* ---- batched sweep: many independent runs in lockstep -------------------- */
+/* ---- batched sweep: many independent runs together ------------------------ */
 /* The reference runs one instance per process; a parameter sweep is many
  * processes.  A batch advances `n` independent runs (each its own context
- * and state, grids of different sizes) by one time step.  Every kernel of
- * the step is launched once for the whole table (each block serves one
- * instance), and the Picard and GMRES loops run in lockstep: each instance
- * keeps its own convergence tests and iteration counts, and an instance that
- * has converged is masked out of the later passes while the others
- * continue.  The step is one CUDA graph (batch-level conditional loops)
- * unless VV_GRAPH=0 at context creation, which drives the same kernels from
- * the host.  All instances must share the precision, bracket scheme and the
+ * and state, grids of different sizes) by one time step.  An instance whose
+ * state fits the shared memory of a thread-block cluster runs its whole step
+ * on one cluster (2 to 16 CTAs by its size), at its own pace; the clusters of
+ * one size are one launch, the costliest instances of the last step first.
+ * The other instances, or all of them under VV_CLUSTER=0 or VV_BATCH_SHAPE,
+ * run as one table in lockstep: every kernel of the step is launched once for
+ * the table, each instance keeps its own convergence tests and iteration
+ * counts, and an instance that has converged is masked out of the later
+ * passes while the others continue.  The table's step is one CUDA graph
+ * (batch-level conditional loops) unless VV_GRAPH=0 at context creation,
+ * which drives the same kernels from the host.  All instances must share the precision, bracket scheme and the
  * tensor_kinetic preconditioner, use the factored order and have nx a
  * multiple of 64; otherwise vv_batch_create returns VV_ERR_UNSUPPORTED.
- * Results equal each instance's own vv_step to rounding (the batch uses the
- * radix-2 x-FFT and 64 x 32 stencil tiles for every instance).  Contexts and
+ * Results equal each instance's own vv_step to rounding.  Contexts and
  * states stay owned by the caller and must outlive the batch. */
 typedef struct vv_batch vv_batch;
 int vv_batch_create(int n, vv_ctx* const* ctxs, const vv_state* states, vv_batch** out);
@@ -428,7 +430,8 @@ int vv_timing_read(vv_ctx* ctx, int64_t* launches, double* total_ms, int reset);
 int vv_launch_count(vv_ctx* ctx, int64_t* launches, int reset);
 /* Kernel variants the context runs, as five ints: FFT kind of the
  * preconditioner's x transforms (0 shared-memory radix-2, 1 four-step
- * register/shuffle, 2 direct DFT), FFT rows per CTA, tridiagonal kind (0 CTA
+ * register/shuffle, 2 direct DFT, 3 the v-major stages: register FFT of
+ * whole rows and overlapping chunks of the v lines), FFT rows per CTA, tridiagonal kind (0 CTA
  * per mode, 1 warp per mode), narrow bracket tiles (1: 32 x 16 instead of
  * 64 x 32) and the marching Jacobian stencil's strip width (0: tiles).
  * vv_create picks them by timing the candidates on the device at hand, or

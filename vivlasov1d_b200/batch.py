@@ -1,25 +1,24 @@
-"""Batched sweep: many independent runs advanced in lockstep.
+"""Batched sweep: many independent runs advanced together.
 
 The reference runs one instance per process (a parameter sweep is many
 ``run.py`` invocations).  ``Batch`` takes several ``Run`` objects -- any mix
 of grid sizes, initial conditions and parameters, each with its own libvv
 context -- and advances all of them by one implicit time step per
-``step()`` call: one CUDA graph in which every kernel serves the whole
-instance table (``vv_batch_step``).  Each instance keeps its own Picard and
-GMRES state and convergence tests; converged instances are masked out of
-later passes while the others continue.
+``step()`` call (``vv_batch_step``).  An instance that fits the shared memory
+of a thread-block cluster runs its whole step there at its own pace; the
+others form a table whose kernels serve all of them in lockstep, in one CUDA
+graph.  Each instance keeps its own Picard and GMRES state and convergence
+tests.
 
-A lockstep pass lasts as long as its slowest instance: in a sweep a few
+A lockstep table's pass lasts as long as its slowest instance: in a sweep a few
 instances need ten times the median's GMRES iterations, and they run with
 few others at the end of every pass.  ``split="auto"`` steps the first call
 as one table and then, for tables of at least ``SPLIT_MIN`` instances,
 re-forms it as two tables -- the eighth of the instances that needed the
 most GMRES iterations, and the rest -- which every later step launches at
 once on two streams (``vv_batch_launch``) and collects together
-(``vv_batch_collect``), so that the two tables' passes interleave.  On the
-256-instance sweep this saves 8% of an FP64 step and costs 1-3% of a
-mixed-precision one: the slow table's instances are the largest, and both
-tables' kernels need the whole GPU.  Each instance computes the same
+(``vv_batch_collect``), so that the two tables' passes interleave.  Instances
+on clusters do not wait for one another and gain nothing by it.  Each instance computes the same
 operations in either form (the tables' tuned kernel shapes may differ, so
 results agree to rounding).
 
@@ -131,7 +130,7 @@ class _Lockstep:
 
 
 class Batch:
-    """Runs advanced together; ``split``: None (one lockstep table), "auto"
+    """Runs advanced together; ``split``: None (one batch), "auto"
     (the first step as one table, then the slowest eighth of the instances
     and the rest as two concurrent tables, for tables of at least
     SPLIT_MIN instances) or a list of index lists (those tables, each run

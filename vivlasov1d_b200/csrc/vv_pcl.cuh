@@ -10,7 +10,7 @@
 //                 chunk takes its carry from the `lev` chunks before it, as in
 //                 vv_cluster.cuh: |l| <= 2 - sqrt(3) but for the 1/ht term, so the
 //                 products of the LU multipliers over lev chunks are below 1e-18
-//                 (1e-10 in FP32; the host finds lev from the multipliers).  The
+//                 (1e-9 in FP32; the host finds lev from the multipliers).  The
 //                 block's first and last lev chunks only provide carries and are
 //                 recomputed by the neighbours: nothing waits on another block,
 //                 at 1 + 2 lev / (TL_WARPS - 2 lev) times the reads.

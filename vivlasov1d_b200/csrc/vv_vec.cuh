@@ -233,7 +233,7 @@ __global__ void k_gm_scale(DevState* s, T* __restrict__ V, size_t ldv, size_t n)
 // GS_Q basis vectors in flight.  The passes stream the basis from HBM or L2;
 // with one value and one vector at a time they ran at the latency of a load per
 // basis vector (256 x 512 FP64 at mean index 15: multi-dot 37 -> 14 us, multi-axpy
-// 61 -> 14; 1024 x 2048 FP32: 46 -> 30 and 87 -> 31 us).
+// 61 -> 14; 1024 x 2048 FP32 over a step: 47 -> 35 and 92 -> 33 us).
 constexpr int GS_Q = 4;
 template <typename T, int VN> struct GsVec { T v[VN]; };
 template <typename T, int VN> VV_DEV GsVec<T, VN> gs_ld(const T* p) {
