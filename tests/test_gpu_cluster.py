@@ -136,3 +136,24 @@ def test_cluster_batch_with_instances_that_do_not_fit(monkeypatch):
         assert _rel(a.fc, b.fc) <= 1e-12
     assert batch.launch_count() > 0
     assert batch.time_kernel(0, it=2, reps=2) > 0
+
+
+@pytest.mark.parametrize("nx,precision", [(64, "fp64"), (256, "fp64"), (50, "fp64"), (64, "mixed")])
+def test_cluster_cta_without_rows(monkeypatch, nx, precision):
+    """100 rows over 16 CTAs of 7: the last CTA owns none and may add nothing
+    to a reduction, whatever its shared memory holds.  A run of 112 rows (same
+    layout, every CTA full) whose f is NaN leaves NaN in every CTA's W and V_0."""
+    from vivlasov1d_b200 import _lib
+    kw = {"rtol": 1e-4} if precision == "mixed" else {}
+    dirty, _, _ = _run(monkeypatch, 16, nx, 112, precision=precision, max_iter=2, **kw)
+    run, _, _ = _run(monkeypatch, 16, nx, 100, precision=precision, **kw)
+    ref, _, _ = _run(monkeypatch, 0, nx, 100, precision=precision, **kw)
+    for _ in range(2):
+        dirty.fc.fill_(float("nan"))
+        with pytest.raises(_lib.VVError):
+            dirty.step()
+        rep = run.step()
+        ref.step()
+        assert rep["ksp_failures"] == 0
+    # in the mixed mode two runs inside the 1e-11 residual ball differ by 2 ht atol a step
+    assert float((run.fc - ref.fc).norm()) <= 2 * 2 * 0.1 * 1e-11 + 1e-12 * float(ref.fc.norm())

@@ -800,9 +800,13 @@ template <typename T, int M> struct ClRun {
     // basis, QU vectors' loads in flight
     template <int NI, int QU> VV_DEV void dots(int m) {
         ClState* S = st();
-        const int E = items(), last = max(E - 1, 0);
+        const int E = items(), last = E - 1;
+        if (E == 0) {   // a CTA past the last row: nothing of its W or V was ever written
+            for (int q = lane(); q < m; q += 32) S->dot[q * CL_WARPS + warp()] = 0.0;
+            return;
+        }
 #pragma unroll 1
-        for (int b = 0; b == 0 || b < E; b += NI * CL_THREADS) {
+        for (int b = 0; b < E; b += NI * CL_THREADS) {
             double w[NI][VN];
             int o[NI];
 #pragma unroll
