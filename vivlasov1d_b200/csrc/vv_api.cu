@@ -2459,18 +2459,19 @@ int vv_create(const vv_grid* grid, vv_ctx** out) {
                 vv_destroy(c);
                 return s;
             }
-            *out = c;
-            return VV_OK;
-        }
-    }
-    {
-        const char* e = getenv("VV_AUTOTUNE");
-        if (!(e && e[0] == '0')) {
-            if ((s = autotune(c)) != VV_OK) {
+        } else {
+            const char* e = getenv("VV_AUTOTUNE");
+            if (!(e && e[0] == '0') && (s = autotune(c)) != VV_OK) {
                 vv_destroy(c);
                 return s;
             }
         }
+    }
+    // the tables are built on the legacy stream: done before the caller's stream,
+    // which may be one that does not wait for it, can read or rewrite them
+    if (cudaStreamSynchronize(c->st) != cudaSuccess) {
+        vv_destroy(c);
+        return fail_cuda(cudaGetLastError(), "vv_create tables");
     }
     *out = c;
     return VV_OK;
