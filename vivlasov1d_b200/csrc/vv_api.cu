@@ -200,6 +200,7 @@ int dalloc(T** p, size_t count) {
     cudaError_t e = cudaMalloc((void**)p, count * sizeof(T));
     if (e != cudaSuccess) {
         *p = nullptr;
+        cudaGetLastError();   // not the next launch's error
         snprintf(g_err, sizeof g_err, "cudaMalloc(%zu bytes): %s", count * sizeof(T), cudaGetErrorString(e));
         return VV_ERR_ALLOC;
     }
@@ -772,7 +773,8 @@ int pcl_apply_t(vv_ctx* c, const TI* X, TO* Y, const int* yidx, int yoff) {
     return launch_irfftl<R, TO>(c, spec2, Y, p);
 }
 
-// tables of the v-major preconditioner (false: it does not apply to this grid)
+// tables of the v-major preconditioner (false: it does not apply to this grid;
+// VV_ERR_ALLOC: no room for them, the former kinds are unaffected)
 int vmaj_prepare(vv_ctx* c, bool* ok) {
     *ok = false;
     if (!vmaj_ok(c) || !c->cl_lf) return VV_OK;
@@ -1647,7 +1649,8 @@ int autotune(vv_ctx* c) {
             c->march = kv.second.march;
             if (kv.second.vmaj && c->g.preconditioner == VV_PC_TENSOR_KINETIC) {
                 bool ok = false;
-                TRY(vmaj_prepare(c, &ok));
+                const int r = vmaj_prepare(c, &ok);
+                if (r != VV_ERR_ALLOC) TRY(r);
                 c->vmaj = ok ? 1 : 0;
             }
             return VV_OK;
@@ -1685,9 +1688,12 @@ int autotune(vv_ctx* c) {
     c->pcR = best.pcR;
     c->tri_kind = best.tri_kind;
     // the v-major stages on grids of 64 K cells and more (below, every variant is at launch latency)
+    bool no_room = false;
     if (c->g.preconditioner == VV_PC_TENSOR_KINETIC && c->ncell >= 65536) {
         bool ok = false;
-        TRY(vmaj_prepare(c, &ok));
+        const int r = vmaj_prepare(c, &ok);
+        no_room = r == VV_ERR_ALLOC;
+        if (!no_room) TRY(r);
         if (ok) {
             c->vmaj = 1;
             float ms = 0.f;
@@ -1744,7 +1750,8 @@ int autotune(vv_ctx* c) {
     }
     c->march = best.march;
     c->launches = 0;
-    tune_cache().push_back({key, best});
+    // without the v-major candidate for want of memory: not the shape's verdict
+    if (!no_room) tune_cache().push_back({key, best});
     return VV_OK;
 }
 
@@ -2441,12 +2448,15 @@ int vv_create(const vv_grid* grid, vv_ctx** out) {
         if (!(sh && sh[0]) && ctas > 0) {
             const vv::ClShape t = vv::cl_shape(nx, nv, c->pow2, ctas, c->mixed ? 4 : 8, vv::cl_smem_limit(c->mixed));
             if (t.ctas && vv::cl_resident(c->mixed, t.fam, t.ctas, t.smem) > 0) {
-                if ((s = cl_prepare(c, t)) != VV_OK) {
+                s = cl_prepare(c, t);
+                if (s != VV_OK && s != VV_ERR_ALLOC) {
                     vv_destroy(c);
                     return s;
                 }
-                c->cls = t;
-                cl_describe(c, t, nullptr, c->cl_host);
+                if (s == VV_OK) {   // no room for its tables: the multi-kernel step
+                    c->cls = t;
+                    cl_describe(c, t, nullptr, c->cl_host);
+                }
             }
         }
     }
@@ -3646,11 +3656,12 @@ int cl_batch_build(vv_batch* b) {
                 if (t.ctas && vv::cl_resident(c->mixed, t.fam, t.ctas, t.smem) < 1) t = vv::ClShape{};
             }
         b->cost[i] = (double)c->ncell;
-        if (!t.ctas) {
+        const int s = t.ctas ? cl_prepare(c, t) : VV_OK;
+        if (s != VV_OK && s != VV_ERR_ALLOC) return s;
+        if (!t.ctas || s == VV_ERR_ALLOC) {
             b->rest_idx.push_back(i);
             continue;
         }
-        TRY(cl_prepare(c, t));
         cl_describe(c, t, &b->states[i], &tab[i]);
         vv_batch::ClClass* k = nullptr;
         for (auto& q : b->classes)
@@ -3719,7 +3730,13 @@ int vv_batch_create(int n, vv_ctx* const* ctxs, const vv_state* states, vv_batch
     b->states.assign(states, states + n);
     b->mixed = ctxs[0]->mixed;
     b->cl = true;
-    auto fail_b = [&](int code) { vv_batch_destroy(b); return code; };
+    // no room for the tables of this kind: the lockstep batch
+    auto fail_b = [&](int code) {
+        vv_batch_destroy(b);
+        if (code != VV_ERR_ALLOC) return code;
+        cudaGetLastError();   // the failed allocation's
+        return lockstep_create(n, ctxs, states, out);
+    };
     int r = cl_batch_build(b);
     if (r != VV_OK) return fail_b(r);
     if (b->classes.empty()) {   // nothing fits
