@@ -3712,6 +3712,35 @@ int cl_batch_launch(vv_batch* b) {
     return VV_OK;
 }
 
+// a step of the batch: the clusters, the lockstep rest beside them, the reports' words
+int cl_batch_enqueue(vv_batch* b, const vv_snes_opts* so, const vv_ksp_opts* ko) {
+    TRY(cl_batch_launch(b));
+    if (b->rest) {
+        b->rest->user = b->rest_st;
+        CK(cudaStreamWaitEvent(b->rest_st, b->fork, 0));
+        TRY(vv_batch_launch(b->rest, so, ko));
+        CK(cudaEventRecord(b->rest_done, b->rest_st));
+        CK(cudaStreamWaitEvent(b->user, b->rest_done, 0));
+    }
+    vv::k_b_gather_states<<<b->n, 128, 0, b->user>>>(b->tab, b->words, b->gather);
+    b->launches++;
+    CK(cudaGetLastError());
+    CK(cudaMemcpyAsync(b->hgather, b->gather, (size_t)b->n * b->words * sizeof(unsigned int), cudaMemcpyDeviceToHost,
+                       b->user));
+    return VV_OK;
+}
+
+// after a step that could only be enqueued in part: wait for what runs, so that
+// the batch is idle (the orders in pinned memory, the states) as its caller is told
+void cl_batch_drain(vv_batch* b) {
+    for (auto& k : b->classes) cudaStreamSynchronize(k.st);
+    if (b->rest) {
+        cudaStreamSynchronize(b->rest_st);
+        b->rest->pending = 0;
+    }
+    cudaStreamSynchronize(b->user);
+}
+
 }  // namespace
 
 extern "C" {
@@ -4015,21 +4044,10 @@ int vv_batch_launch(vv_batch* b, const vv_snes_opts* so, const vv_ksp_opts* ko) 
     b->st = b->user;
     b->pending_l0 = b->launches;
     if (b->cl) {
-        TRY(cl_batch_launch(b));
-        if (b->rest) {   // beside the clusters
-            b->rest->user = b->rest_st;
-            CK(cudaStreamWaitEvent(b->rest_st, b->fork, 0));
-            TRY(vv_batch_launch(b->rest, so, ko));
-            CK(cudaEventRecord(b->rest_done, b->rest_st));
-            CK(cudaStreamWaitEvent(b->user, b->rest_done, 0));
-        }
-        vv::k_b_gather_states<<<b->n, 128, 0, b->user>>>(b->tab, b->words, b->gather);
-        b->launches++;
-        CK(cudaGetLastError());
-        CK(cudaMemcpyAsync(b->hgather, b->gather, (size_t)b->n * b->words * sizeof(unsigned int),
-                           cudaMemcpyDeviceToHost, b->user));
-        b->pending = 1;
-        return VV_OK;
+        const int r = cl_batch_enqueue(b, so, ko);
+        if (r != VV_OK) cl_batch_drain(b);
+        b->pending = r == VV_OK;
+        return r;
     }
     CK(cudaMemsetAsync(b->counts, 0, vv::BN_WORDS * sizeof(unsigned int), b->user));
     if (b->use_graph) {
@@ -4055,6 +4073,7 @@ int vv_batch_collect(vv_batch* b, const vv_snes_opts* so, const vv_ksp_opts* ko,
                      int* statuses) {
     if (!b || !so || !ko || !reports) return VV_ERR_ARG;
     if (!b->pending) return fail(VV_ERR_ARG, "vv_batch_collect: nothing launched");
+    const cudaError_t done = cudaStreamSynchronize(b->user);   // the whole step, the rest's included
     b->pending = 0;
     if (b->rest) {
         const int r = vv_batch_collect(b->rest, so, ko, b->rest_rep.data(), b->rest_status.data());
@@ -4062,7 +4081,7 @@ int vv_batch_collect(vv_batch* b, const vv_snes_opts* so, const vv_ksp_opts* ko,
         b->launches += b->rest->launches;
         b->rest->launches = 0;
     }
-    CK(cudaStreamSynchronize(b->user));
+    CK(done);
     if (b->use_graph) {
         const unsigned* k = b->hcounts;
         b->launches = b->pending_l0 + 1 + b->nk_prologue + b->nk_revert_ctrl +
