@@ -157,3 +157,26 @@ def test_cluster_cta_without_rows(monkeypatch, nx, precision):
         assert rep["ksp_failures"] == 0
     # in the mixed mode two runs inside the 1e-11 residual ball differ by 2 ht atol a step
     assert float((run.fc - ref.fc).norm()) <= 2 * 2 * 0.1 * 1e-11 + 1e-12 * float(ref.fc.norm())
+
+
+@pytest.mark.parametrize("bad", ["diverged", "nan"])
+def test_cluster_batch_isolates_a_failing_instance(monkeypatch, bad):
+    """A failing instance (f scaled until the residual passes 10, or NaN in f)
+    between others of its cluster class and of another: it alone reports it, and
+    the others' f equal those of a batch without it, bit for bit."""
+    from vivlasov1d_b200 import _lib
+    from vivlasov1d_b200.batch import Batch
+    sizes = [(64, 128), (64, 200), (64, 100), (128, 256)]
+    runs, ref = ([_run(monkeypatch, 16, *s, max_it=100)[0] for s in sizes] for _ in range(2))
+    if bad == "nan":
+        runs[1].fc[9, 5] = float("nan")
+    else:
+        runs[1].fc.mul_(1e3)
+        runs[1].calculate_moments()
+    want = _lib.VV_ERR_NAN if bad == "nan" else _lib.VV_ERR_DIVERGED
+    b, bref = Batch(runs), Batch([ref[i] for i in (0, 2, 3)])
+    for _ in range(2):
+        reps, rref = b.step(), bref.step()
+        assert [r["status"] for r in reps] == [_lib.VV_OK, want, _lib.VV_OK, _lib.VV_OK]
+        for i, q in zip((0, 2, 3), rref):
+            assert reps[i]["gmres_its"] == q["gmres_its"] and torch.equal(runs[i].fc, ref[i].fc)
