@@ -422,7 +422,10 @@ int vv_invariants(vv_ctx* ctx, const double* f, const double* phi, const double*
 /* ---- timing of the dominant kernel (measurement support) --------------- */
 /* When enabled, the library records CUDA events around every launch of the
  * Jacobian-vector-product stencil kernel on its stream; vv_timing_read
- * returns the number of launches and their summed device time (ms). */
+ * returns the number of launches and their summed device time (ms).  While it
+ * is enabled, vv_step and vv_gmres run the multi-kernel path driven from the
+ * host, where that stencil is a launch of its own (inside a step's graph or on
+ * a thread-block cluster it is not). */
 int vv_timing_enable(vv_ctx* ctx, int enable);
 int vv_timing_read(vv_ctx* ctx, int64_t* launches, double* total_ms, int reset);
 /* Number of kernels the library has launched since the last reset

@@ -180,3 +180,30 @@ def test_cluster_batch_isolates_a_failing_instance(monkeypatch, bad):
         assert [r["status"] for r in reps] == [_lib.VV_OK, want, _lib.VV_OK, _lib.VV_OK]
         for i, q in zip((0, 2, 3), rref):
             assert reps[i]["gmres_its"] == q["gmres_its"] and torch.equal(runs[i].fc, ref[i].fc)
+
+
+@pytest.mark.parametrize("ctas", [16, 0])
+def test_timing_counts_the_stencil_of_steps_and_solves(monkeypatch, ctas):
+    """Timing enabled: one timed launch of the Jacobian stencil per GMRES
+    iteration at least, in a step and in a solve, wherever they run without it."""
+    import ctypes as C
+    from vivlasov1d_b200 import _lib
+    run, _, _ = _run(monkeypatch, ctas, 64, 130)
+    plain, _, _ = _run(monkeypatch, ctas, 64, 130)
+    run.step(), plain.step()
+    run.ctx.timing_enable(True)
+    its = sum(run.step()["gmres_its"])
+    n, ms = run.ctx.timing_read()
+    assert its > 0 and n >= its and ms > 0
+    b, x = run.fc.clone(), torch.empty_like(run.fc)
+    o = _lib.vv_ksp_opts(rtol=1e-9, atol=1e-50, dtol=1e5, max_it=400, restart=0)
+    r = _lib.vv_ksp_result()
+    run.ctx.call("vv_gmres", run.ctx.field(b), run.ctx.field(x), C.byref(o), C.byref(r))
+    n, ms = run.ctx.timing_read()
+    assert r.its > 0 and n >= r.its and ms > 0
+    run.ctx.timing_enable(False)
+    run.step()
+    assert run.ctx.timing_read()[0] == 0
+    for _ in range(2):
+        plain.step()
+    assert _rel(run.fc, plain.fc) <= 1e-12

@@ -116,7 +116,7 @@ struct vv_ctx {
     size_t smem_rfft, smem_irfft, smem_tri, smem_pois;
     bool tri_stage;
     bool pivot_differs;
-    // timing of the JVP stencil kernel (host-driven path)
+    // timing of the JVP stencil kernel (the steps and solves are host-driven then)
     bool timing;
     std::vector<cudaEvent_t> ev;
     size_t ev_used;
@@ -1848,7 +1848,7 @@ int build_step_graph(vv_ctx* c, vv_state* st) {
 
 // Read the step report of context c from its pinned state copy.
 int fill_report(vv_ctx* c, const vv::DevState& d, int restart, vv_step_report* rep, double abort_residual,
-                bool count_launches = true) {
+                bool graph) {
     std::memset(rep, 0, sizeof(*rep));
     rep->picard_its = d.pic_i;
     rep->gmres_its_total = d.gmres_total;
@@ -1867,7 +1867,7 @@ int fill_report(vv_ctx* c, const vv::DevState& d, int restart, vv_step_report* r
         rep->guess_residual = d.guess_res;
     }
     (void)restart;
-    if (c->use_graph && count_launches) {
+    if (graph) {
         // kernels the graph executed: top level once, the Picard body per pass,
         // the GMRES cycle body per cycle (+ restart branch), the Arnoldi body per iteration
         const int64_t top = c->nk_top - c->nk_pic - c->nk_revert;
@@ -2658,7 +2658,8 @@ int vv_gmres(vv_ctx* c, const double* b, double* x, const vv_ksp_opts* o, vv_ksp
     c->opts_valid = false;
     for (int k = 0; k < 5; ++k) c->hnd[k] = saved[k];
     TRY(s);
-    if (c->cls.ctas && restart <= vv::CL_RESTART && (c->mixed || (aligned16(b) && aligned16(x) && b != x))) {
+    if (c->cls.ctas && restart <= vv::CL_RESTART && !c->timing &&
+        (c->mixed || (aligned16(b) && aligned16(x) && b != x))) {
         if (c->mixed) {
             vv::k_scale<double, float><<<grid1d(c->ncell, 256), 256, 0, c->st>>>(b, c->bvec32, c->ncell, nullptr, 1.0);
             CKL(c);
@@ -2810,12 +2811,14 @@ int vv_step(vv_ctx* c, vv_state* st, const vv_snes_opts* so, const vv_ksp_opts* 
         c->coll_p = {st->n, st->u, st->a};
     }
     std::memset(rep, 0, sizeof(*rep));
-    const bool cluster = c->cls.ctas && restart <= vv::CL_RESTART;
+    // with timing enabled the host drives the step: the timed kernel is a launch of its own there
+    const bool cluster = c->cls.ctas && restart <= vv::CL_RESTART && !c->timing;
+    const bool graph = !cluster && c->use_graph && !c->timing;
     if (cluster) {
         for (auto& h : c->hnd) h = 0;
         TRY(upload_options(c, ko, so));
         TRY(cl_run_single(c, st, nullptr, nullptr));
-    } else if (c->use_graph) {
+    } else if (graph) {
         if (!c->step_exec || !same_state(c->step_key, *st)) TRY(build_step_graph(c, st));
         std::memcpy(c->hnd, c->step_hnd, sizeof c->hnd);
         TRY(upload_options(c, ko, so));
@@ -2831,7 +2834,7 @@ int vv_step(vv_ctx* c, vv_state* st, const vv_snes_opts* so, const vv_ksp_opts* 
     // report
     CK(cudaMemcpyAsync(c->hds, c->ds, offsetof(vv::DevState, hcol), cudaMemcpyDeviceToHost, c->st));
     CK(cudaStreamSynchronize(c->st));
-    return fill_report(c, *c->hds, restart, rep, so->abort_residual, !cluster);
+    return fill_report(c, *c->hds, restart, rep, so->abort_residual, graph);
 }
 
 int vv_invariants(vv_ctx* c, const double* f, const double* phi, const double* h2, vv_invariant_set* out) {
