@@ -431,7 +431,9 @@ int vv_timing_read(vv_ctx* ctx, int64_t* launches, double* total_ms, int reset);
 /* Number of kernels the library has launched since the last reset
  * (kernels executed inside the time-step graph included). */
 int vv_launch_count(vv_ctx* ctx, int64_t* launches, int reset);
-/* Kernel variants the context runs, as five ints: FFT kind of the
+/* Variants of the context's separate kernels (the preconditioner and stencil
+ * calls, and the steps and solves that do not run on a thread-block cluster;
+ * those that do have one kernel), as five ints: FFT kind of the
  * preconditioner's x transforms (0 shared-memory radix-2, 1 four-step
  * register/shuffle, 2 direct DFT, 3 the v-major stages: register FFT of
  * whole rows and overlapping chunks of the v lines), FFT rows per CTA, tridiagonal kind (0 CTA
