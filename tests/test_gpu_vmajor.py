@@ -84,3 +84,17 @@ def test_gram_schmidt_passes(monkeypatch, nx, nv, restart):
     y = grid.field()
     s.jacobian(x.clone(), y)
     assert float((b - y).norm()) <= 1.01 * rnorm + 1e-9 * float(b.norm())
+
+
+def test_variants_are_tuned_per_overlap():
+    """The v-major stages' overlap follows from ht: a choice timed at one ht is
+    not taken over at another.  A context that takes its variants from the cache
+    launches one kernel in its constructor (the table), a timed one reports none."""
+    from vivlasov1d_b200.solver import Grid
+    counts = []
+    for ht in (0.05, 0.05, 1e-6):
+        ctx = Grid(1024, 1031, 4 * np.pi, 8.0, ht=ht).context(bracket="arakawaj4", preconditioner="tensor_kinetic")
+        if ht == 0.05:
+            assert ctx.kernel_shape()[0] == 3
+        counts.append(ctx.launch_count())
+    assert counts == [0, 1, 0]

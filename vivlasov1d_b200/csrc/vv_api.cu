@@ -773,11 +773,8 @@ int pcl_apply_t(vv_ctx* c, const TI* X, TO* Y, const int* yidx, int yoff) {
     return launch_irfftl<R, TO>(c, spec2, Y, p);
 }
 
-// tables of the v-major preconditioner (false: it does not apply to this grid;
-// VV_ERR_ALLOC: no room for them, the former kinds are unaffected)
-int vmaj_prepare(vv_ctx* c, bool* ok) {
-    *ok = false;
-    if (!vmaj_ok(c) || !c->cl_lf) return VV_OK;
+// carry levels of the v-major solves, from the context's multipliers
+void vmaj_levels(vv_ctx* c) {
     // chunks after which every product of the multipliers is negligible (both sweeps)
     const double tol = c->mixed ? 1e-9 : 1e-18;
     auto levels = [&](int ch) {
@@ -798,6 +795,14 @@ int vmaj_prepare(vv_ctx* c, bool* ok) {
     };
     c->vm_lev16 = levels(16);
     c->vm_lev8 = levels(8);
+}
+
+// tables of the v-major preconditioner (false: it does not apply to this grid;
+// VV_ERR_ALLOC: no room for them, the former kinds are unaffected)
+int vmaj_prepare(vv_ctx* c, bool* ok) {
+    *ok = false;
+    if (!vmaj_ok(c) || !c->cl_lf) return VV_OK;
+    if (c->vm_lev16 == 0) vmaj_levels(c);
     if (vv::TL_WARPS - 2 * c->vm_lev16 <= 0 && vv::TL_WARPS - 2 * c->vm_lev8 <= 0) return VV_OK;
     const size_t cnt = (size_t)c->nmodes * c->nv, csz = c->mixed ? sizeof(float2) : sizeof(double2);
     if (!c->vm_dinv) {
@@ -1609,13 +1614,15 @@ bool same_state(const vv_state& a, const vv_state& b) { return std::memcmp(&a, &
 // scratch buffers (CUDA events, a few launches each) and keeps the fastest:
 // FFT kind x rows per CTA x tridiagonal kind for the preconditioner in the
 // GMRES precision, and the bracket tile shape.  Results are cached per
-// (nx, nv, precision, time derivative, preconditioner) for the life of the process.
+// (nx, nv, precision, time derivative, preconditioner, carry levels of the
+// v-major stages: they follow from ht and hv and set those stages' overlap) for
+// the life of the process.
 struct TuneResult {
     int fft_kind, pcR, tri_kind, narrow, march, vmaj;
 };
 
-std::vector<std::pair<std::array<int, 5>, TuneResult>>& tune_cache() {
-    static std::vector<std::pair<std::array<int, 5>, TuneResult>> cache;
+std::vector<std::pair<std::array<int, 7>, TuneResult>>& tune_cache() {
+    static std::vector<std::pair<std::array<int, 7>, TuneResult>> cache;
     return cache;
 }
 
@@ -1639,7 +1646,11 @@ int time_it(vv_ctx* c, F fn, int reps, float* ms) {
 }
 
 int autotune(vv_ctx* c) {
-    const std::array<int, 5> key = {c->nx, c->nv, c->mixed ? 1 : 0, c->avg, c->g.preconditioner};
+    // the v-major stages are a candidate from 64 K cells on (below, every variant is at launch latency)
+    const bool vmaj = c->g.preconditioner == VV_PC_TENSOR_KINETIC && c->ncell >= 65536 && vmaj_ok(c);
+    if (vmaj) vmaj_levels(c);
+    const std::array<int, 7> key = {c->nx, c->nv, c->mixed ? 1 : 0, c->avg, c->g.preconditioner,
+                                    vmaj ? c->vm_lev16 : 0, vmaj ? c->vm_lev8 : 0};
     for (auto& kv : tune_cache())
         if (kv.first == key) {
             c->fft_kind = kv.second.fft_kind;
@@ -1647,7 +1658,7 @@ int autotune(vv_ctx* c) {
             c->tri_kind = kv.second.tri_kind;
             c->narrow_bracket = kv.second.narrow;
             c->march = kv.second.march;
-            if (kv.second.vmaj && c->g.preconditioner == VV_PC_TENSOR_KINETIC) {
+            if (kv.second.vmaj) {
                 bool ok = false;
                 const int r = vmaj_prepare(c, &ok);
                 if (r != VV_ERR_ALLOC) TRY(r);
@@ -1687,9 +1698,8 @@ int autotune(vv_ctx* c) {
     c->fft_kind = best.fft_kind;
     c->pcR = best.pcR;
     c->tri_kind = best.tri_kind;
-    // the v-major stages on grids of 64 K cells and more (below, every variant is at launch latency)
     bool no_room = false;
-    if (c->g.preconditioner == VV_PC_TENSOR_KINETIC && c->ncell >= 65536) {
+    if (vmaj) {
         bool ok = false;
         const int r = vmaj_prepare(c, &ok);
         no_room = r == VV_ERR_ALLOC;
