@@ -78,7 +78,7 @@ struct vv_ctx {
     float2 *twv32, *pv_spec32;
     float* pv_xt32;
     cudaStream_t st;      // the caller's stream
-    int device;
+    int device, nsm;      // nsm: its SMs
     // device buffers
     double *v, *h0, *hxp, *Fh, *tmp, *bvec, *delta, *fl, *V, *part, *scal, *xscratch, *mom_part;
     double2 *spec, *tw, *lambda, *dinv;
@@ -286,11 +286,10 @@ template <int SCHEME, typename T, int MW>
 int launch_march(vv_ctx* c, const T* X, T* Y, const vv::BracketParams& p) {
     const size_t smem = vv::MarchRow<T, MW>::smem_bytes();
     constexpr int CH = vv::MarchShape<T>::CH;
-    int per_sm = 0, nsm = 148;
+    int per_sm = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, vv::k_bracket_march<SCHEME, T, MW>, MW, smem);
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device);
     const int strips = c->nx / MW;
-    const long target = 2L * nsm * std::max(1, per_sm);
+    const long target = 2L * c->nsm * std::max(1, per_sm);
     const int nseg = (int)std::max<long>(1, (target + strips - 1) / strips);
     int seg = (c->nv + nseg - 1) / nseg;
     seg = std::max(CH, (seg + CH - 1) / CH * CH);
@@ -758,7 +757,7 @@ int pcl_apply_t(vv_ctx* c, const TI* X, TO* Y, const int* yidx, int yoff) {
     // chunks of 16 rows, of 8 (twice the blocks, more overlap) where those are fewer than the SMs
     const int tiles = (c->nmodes + 31) / 32, u16 = (vv::TL_WARPS - 2 * c->vm_lev16) * 16;
     const int u8 = (vv::TL_WARPS - 2 * c->vm_lev8) * 8;
-    const bool small = u8 > 0 && (u16 <= 0 || tiles * ((c->nv + u16 - 1) / u16) < 148);
+    const bool small = u8 > 0 && (u16 <= 0 || tiles * ((c->nv + u16 - 1) / u16) < c->nsm);
     const int un = small ? u8 : u16;
     const dim3 g((unsigned)tiles, (unsigned)((c->nv + un - 1) / un));
     const C2* dj = reinterpret_cast<const C2*>(c->vm_dinv);
@@ -2097,6 +2096,8 @@ int vv_create(const vv_grid* grid, vv_ctx** out) {
     c->ncell = (size_t)g.nx * g.nv;
     c->st = 0;
     cudaGetDevice(&c->device);
+    c->nsm = 148;
+    cudaDeviceGetAttribute(&c->nsm, cudaDevAttrMultiProcessorCount, c->device);
     {
         const char* e = getenv("VV_GRAPH");
         c->use_graph = !(e && e[0] == '0');
