@@ -423,6 +423,10 @@ __global__ void k_irfft4(const typename Cplx<R>::type* __restrict__ spec, TO* __
 // sum and difference are staged).  With fewer than eight tiles of modes the
 // sum over n is split over the warps.  201 x 401 in FP64: forward 8.5 us,
 // inverse 9.2 us, the function call that holds them 49 -> 28.7 us.
+// With one tile (nx < 64) a warp takes one row instead: there the split's
+// barrier and sums cost more than the few products it spreads (whole FP64
+// preconditioner, 152 v rows: nx 17 9.26 -> 7.8 us, nx 56 9.99 -> 9.2; each
+// row's sum halved over two warps: 8.0 and 9.3).
 // ---------------------------------------------------------------------------
 constexpr int DFT_ROWS = 4, DFT_THREADS = 256, DFT_WARPS = DFT_THREADS / 32;
 
@@ -453,6 +457,24 @@ VV_DEV void dft_join(C (&v)[DFT_ROWS], const DftSplit& s, C* red) {
 #pragma unroll
             for (int r = 0; r < DFT_ROWS; ++r)
                 v[r] = c_add(v[r], red[(((q - 1) * s.nT + s.tile) * DFT_ROWS + r) * 32 + lane]);
+    }
+}
+
+// v_r += sum over [na, nb) of (Re x Re w, Im x Im w), w = W^{n kk}, x row r's entry n (RW rows)
+template <int RW, typename C>
+VV_DEV void dft_sums(C (&v)[RW], const C* xs, int nm, const C* stw, int N, int kk, int na, int nb) {
+    int idx = kk * na % N;
+#pragma unroll 2
+    for (int n = na; n < nb; ++n) {
+        const C w = stw[idx];
+#pragma unroll
+        for (int r = 0; r < RW; ++r) {
+            const C x = xs[r * nm + n];
+            v[r].x += x.x * w.x;
+            v[r].y += x.y * w.y;
+        }
+        idx += kk;
+        if (idx >= N) idx -= N;
     }
 }
 
@@ -493,6 +515,15 @@ k_rdft_rows(const TI* __restrict__ X, typename Cplx<R>::type* __restrict__ spec,
         xs[r * nm + n] = v;
     }
     __syncthreads();
+    if (nm <= 32) {   // one tile: a warp one row
+        const int r = threadIdx.x >> 5, k = threadIdx.x & 31, kk = k < nm ? k : 0;
+        if (r >= DFT_ROWS || j0 + r >= p.nv) return;
+        const C e = xs[r * nm];
+        C v[1] = {c_make<C>((double)(e.x + ((kk & 1) ? -e.y : e.y)), 0.0)};
+        dft_sums(v, xs + r * nm, nm, stw, N, kk, 1, half + 1);
+        if (k < nm) spec[(size_t)k * p.nv + j0 + r] = v[0];
+        return;
+    }
     const DftSplit s(nm);
     for (int tile = s.tile; tile < s.nT; tile += s.step) {
         const int k = tile * 32 + (threadIdx.x & 31), kk = k < nm ? k : 0;
@@ -505,19 +536,7 @@ k_rdft_rows(const TI* __restrict__ X, typename Cplx<R>::type* __restrict__ spec,
         }
         if (s.part < s.parts) {
             const int na = 1 + s.part * half / s.parts, nb = 1 + (s.part + 1) * half / s.parts;
-            int idx = (int)((long long)kk * na % N);
-#pragma unroll 2
-            for (int n = na; n < nb; ++n) {
-                const C w = stw[idx];
-#pragma unroll
-                for (int r = 0; r < DFT_ROWS; ++r) {
-                    const C x = xs[r * nm + n];
-                    v[r].x += x.x * w.x;
-                    v[r].y += x.y * w.y;
-                }
-                idx += kk;
-                if (idx >= N) idx -= N;
-            }
+            dft_sums(v, xs, nm, stw, N, kk, na, nb);
         }
         dft_join(v, s, red);
         if (s.part == 0 && k < nm) {
@@ -549,6 +568,24 @@ k_irdft_rows(const typename Cplx<R>::type* __restrict__ spec, TO* __restrict__ Y
     }
     __syncthreads();
     const R inv = (R)(1.0 / (double)N);
+    // samples n and N - n of row r from the sums t
+    auto put = [&](int r, int n, C t) {
+        const C* xr = xs + r * nm;
+        R e = xr[0].x;
+        if (!(N & 1)) e += (n & 1) ? -xr[N / 2].x : xr[N / 2].x;
+        TO* row = Y + (COLS ? (size_t)(j0 + r) : (size_t)(j0 + r) * N);
+        const size_t es = COLS ? (size_t)cols : 1;
+        row[n * es] = (TO)((e + (R)2 * (t.x + t.y)) * inv);
+        if (n > 0 && 2 * n != N) row[(N - n) * es] = (TO)((e + (R)2 * (t.x - t.y)) * inv);
+    };
+    if (nm <= 32) {
+        const int r = threadIdx.x >> 5, n = threadIdx.x & 31;
+        if (r >= DFT_ROWS || j0 + r >= p.nv) return;
+        C v[1] = {c_make<C>(0.0, 0.0)};
+        dft_sums(v, xs + r * nm, nm, stw, N, n < nm ? n : 0, 1, K + 1);
+        if (n < nm) put(r, n, v[0]);
+        return;
+    }
     const DftSplit s(nm);
     for (int tile = s.tile; tile < s.nT; tile += s.step) {
         const int n = tile * 32 + (threadIdx.x & 31), nn = n < nm ? n : 0;
@@ -556,34 +593,15 @@ k_irdft_rows(const typename Cplx<R>::type* __restrict__ spec, TO* __restrict__ Y
 #pragma unroll
         for (int r = 0; r < DFT_ROWS; ++r) v[r].x = v[r].y = R(0);
         if (s.part < s.parts) {
+            // W^{nk} = (cos, -sin): Re(X e^{+i theta}) = X.x w.x + X.y w.y
             const int ka = 1 + s.part * K / s.parts, kb = 1 + (s.part + 1) * K / s.parts;
-            int idx = (int)((long long)nn * ka % N);
-#pragma unroll 2
-            for (int k = ka; k < kb; ++k) {
-                const C w = stw[idx];   // W^{nk} = (cos, -sin): Re(X e^{+i theta}) = X.x w.x + X.y w.y
-#pragma unroll
-                for (int r = 0; r < DFT_ROWS; ++r) {
-                    const C x = xs[r * nm + k];
-                    v[r].x += x.x * w.x;
-                    v[r].y += x.y * w.y;
-                }
-                idx += nn;
-                if (idx >= N) idx -= N;
-            }
+            dft_sums(v, xs, nm, stw, N, nn, ka, kb);
         }
         dft_join(v, s, red);
         if (s.part == 0 && n < nm) {
 #pragma unroll
             for (int r = 0; r < DFT_ROWS; ++r)
-                if (j0 + r < p.nv) {
-                    const C* xr = xs + r * nm;
-                    R e = xr[0].x;
-                    if (!(N & 1)) e += (n & 1) ? -xr[N / 2].x : xr[N / 2].x;
-                    TO* row = Y + (COLS ? (size_t)(j0 + r) : (size_t)(j0 + r) * N);
-                    const size_t es = COLS ? (size_t)cols : 1;
-                    row[n * es] = (TO)((e + (R)2 * (v[r].x + v[r].y)) * inv);
-                    if (n > 0 && 2 * n != N) row[(N - n) * es] = (TO)((e + (R)2 * (v[r].x - v[r].y)) * inv);
-                }
+                if (j0 + r < p.nv) put(r, n, v[r]);
         }
     }
 }
