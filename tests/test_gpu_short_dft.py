@@ -52,3 +52,18 @@ def test_short_rows_mixed_step(monkeypatch, nx, nv):
     ra, rb = a.step(), b.step()
     assert ra["residual"][-1] < 1e-11 and rb["residual"][-1] < 1e-11
     assert float((a.fc - b.fc).norm()) <= 2 * 0.1 * 1e-11 + 1e-12 * float(b.fc.norm())
+
+
+@pytest.mark.parametrize("nx", [4417, 4600, 4735])
+def test_longest_direct_rows(nx):
+    """The longest rows whose twiddles and four rows fit a block's shared memory
+    (48 nx bytes of 227,312).  A row's sums of nx products round to some
+    sqrt(nx) 1.1e-16 < 1e-14 of its size: 1e-12 as for the short rows."""
+    from vivlasov1d_b200.solver import Grid, TensorProductPreconditioner
+    nv = 6
+    x = np.random.default_rng(nx).standard_normal((nx, nv))
+    og, grid = vo.Grid(nx, nv, 4 * np.pi, 8.0, ht=0.05), Grid(nx, nv, 4 * np.pi, 8.0, ht=0.05)
+    X, Y = torch.from_numpy(vo.to_flat(x)).cuda(), grid.field()
+    TensorProductPreconditioner.create("tensor_kinetic", grid=grid).tensorProduct(X, Y)
+    want = vo.TensorKineticPreconditioner(og).apply(x)
+    assert np.abs(vo.from_flat(Y.cpu().numpy()) - want).max() <= 1e-12 * np.abs(want).max()

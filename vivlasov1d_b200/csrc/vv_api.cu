@@ -637,27 +637,6 @@ int raise_smem_limits(int* limit_out) {
         smem_attributes<double>(optin, lowest, e);
         smem_attributes<float>(optin, lowest, e);
         smem_set((const void*)vv::k_moments_poisson, optin, lowest, e);
-#define VV_SETL(M)                                                          \
-    smem_set((const void*)vv::k_rfftl<double, double, M>, optin, lowest, e);  \
-    smem_set((const void*)vv::k_rfftl<double, float, M>, optin, lowest, e);   \
-    smem_set((const void*)vv::k_rfftl<float, float, M>, optin, lowest, e);    \
-    smem_set((const void*)vv::k_irfftl<double, double, M>, optin, lowest, e); \
-    smem_set((const void*)vv::k_irfftl<float, float, M>, optin, lowest, e);
-        VV_SETL(512) VV_SETL(1024) VV_SETL(2048)
-#undef VV_SETL
-#define VV_SETT(R, A)                                                \
-    smem_set((const void*)vv::k_tridiagl<R, A, 8>, optin, lowest, e);  \
-    smem_set((const void*)vv::k_tridiagl<R, A, 16>, optin, lowest, e);
-        VV_SETT(double, false) VV_SETT(double, true) VV_SETT(float, false)
-#undef VV_SETT
-#define VV_SETJ1(M)                                                          \
-    smem_set((const void*)vv::k_rfftj1<double, double, M>, optin, lowest, e);  \
-    smem_set((const void*)vv::k_rfftj1<double, float, M>, optin, lowest, e);   \
-    smem_set((const void*)vv::k_rfftj1<float, float, M>, optin, lowest, e);    \
-    smem_set((const void*)vv::k_irfftj1<double, double, M>, optin, lowest, e); \
-    smem_set((const void*)vv::k_irfftj1<float, float, M>, optin, lowest, e);
-        VV_SETJ1(32) VV_SETJ1(64) VV_SETJ1(128) VV_SETJ1(256)
-#undef VV_SETJ1
         smem_set((const void*)vv::k_b_moments_poisson, optin, lowest, e);
         smem_set((const void*)vv::k_adj_poisson, optin, lowest, e);
 #define VV_SET_MARCH(S)                                                              \
@@ -737,6 +716,48 @@ int launch_irfftl(vv_ctx* c, const typename Cplx<R>::type* spec, TO* Y, const vv
     return VV_OK;
 }
 
+// dynamic shared memory of the kernels that this context's v-major stages launch
+// (apart from raise_smem_limits: the solves' static arrays would lower the limit
+// that holds for every other kernel, and most contexts launch none of them)
+cudaError_t vmaj_attributes(const vv_ctx* c) {
+    cudaError_t e = cudaSuccess;
+    auto set = [&](const void* f, size_t bytes) {
+        if (e == cudaSuccess && bytes > 48 * 1024)
+            e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    };
+    auto rows = [&](const void* d, const void* df, const void* ff, const void* id, const void* iff, size_t slots) {
+        if (c->mixed) {
+            for (const void* f : {df, ff, iff}) set(f, slots * sizeof(float2));
+        } else {
+            for (const void* f : {d, id}) set(f, slots * sizeof(double2));
+        }
+    };
+#define VV_ROWS(K, IK, M_, SLOTS)                                                                           \
+    case M_:                                                                                                \
+        rows((const void*)vv::K<double, double, M_>, (const void*)vv::K<double, float, M_>,                 \
+             (const void*)vv::K<float, float, M_>, (const void*)vv::IK<double, double, M_>,                 \
+             (const void*)vv::IK<float, float, M_>, SLOTS);                                                 \
+        break;
+#define VV_L(M_) VV_ROWS(k_rfftl, k_irfftl, M_, vv::fl_smem(M_, 1))
+#define VV_J(M_) VV_ROWS(k_rfftj1, k_irfftj1, M_, (size_t)vv::fj_slots_of(M_))
+    switch (c->M) {
+        VV_J(32) VV_J(64) VV_J(128) VV_J(256) VV_L(512) VV_L(1024) VV_L(2048)
+    }
+#undef VV_L
+#undef VV_J
+#undef VV_ROWS
+    if (c->mixed) {
+        set((const void*)vv::k_tridiagl<float, false, 8>, vv::tl_smem<float>(8));
+        set((const void*)vv::k_tridiagl<float, false, 16>, vv::tl_smem<float>(16));
+    } else {
+        set((const void*)vv::k_tridiagl<double, false, 8>, vv::tl_smem<double>(8));
+        set((const void*)vv::k_tridiagl<double, false, 16>, vv::tl_smem<double>(16));
+        set((const void*)vv::k_tridiagl<double, true, 8>, vv::tl_smem<double>(8));
+        set((const void*)vv::k_tridiagl<double, true, 16>, vv::tl_smem<double>(16));
+    }
+    return e;
+}
+
 // P^-1 (ADJ: P^-T) through the v-major stages, in the context's GMRES precision
 template <typename TI, typename R, typename TO, bool ADJ>
 int pcl_apply_t(vv_ctx* c, const TI* X, TO* Y, const int* yidx, int yoff) {
@@ -803,6 +824,12 @@ int vmaj_prepare(vv_ctx* c, bool* ok) {
     if (!vmaj_ok(c) || !c->cl_lf) return VV_OK;
     if (c->vm_lev16 == 0) vmaj_levels(c);
     if (vv::TL_WARPS - 2 * c->vm_lev16 <= 0 && vv::TL_WARPS - 2 * c->vm_lev8 <= 0) return VV_OK;
+    const cudaError_t e = vmaj_attributes(c);
+    if (e == cudaErrorMemoryAllocation) {   // no room to load them
+        cudaGetLastError();
+        return VV_ERR_ALLOC;
+    }
+    if (e != cudaSuccess) return fail_cuda(e, "cudaFuncSetAttribute (v-major stages)");
     const size_t cnt = (size_t)c->nmodes * c->nv, csz = c->mixed ? sizeof(float2) : sizeof(double2);
     if (!c->vm_dinv) {
         char* base = nullptr;
