@@ -2260,9 +2260,11 @@ int vv_create(const vv_grid* grid, vv_ctx** out) {
     }
     std::vector<double2> dinv((size_t)nm * nv);
     std::vector<double2> lam2(nm);
+    std::vector<double> mult(nv, 0.0);   // max over the modes of |lambda / U_r|^2
     bool piv = false;
     for (int k = 0; k < nm; ++k) {
         const cd L = lam[k];
+        const double l2 = std::norm(L);
         lam2[k] = make_double2(L.real(), L.imag());
         cd dprev;
         for (int r = 0; r < nv; ++r) {
@@ -2284,6 +2286,7 @@ int vv_create(const vv_grid* grid, vv_ctx** out) {
             }
             const cd di = 1.0 / d;
             dinv[(size_t)k * nv + r] = make_double2(di.real(), di.imag());
+            mult[r] = std::max(mult[r], l2 * std::norm(di));
             dprev = d;
         }
     }
@@ -2450,12 +2453,6 @@ int vv_create(const vv_grid* grid, vv_ctx** out) {
     }
     if (g.preconditioner == VV_PC_TENSOR_KINETIC) {
         // |l_j| = |lambda alpha_j / U_{j-1}|, |m_j| = |lambda gamma_j / U_j|
-        std::vector<double> mult(nv, 0.0);   // max over the modes of |lambda / U_j|^2
-        for (int k = 0; k < nm; ++k) {
-            const double l2 = lam2[k].x * lam2[k].x + lam2[k].y * lam2[k].y;
-            const double2* d = dinv.data() + (size_t)k * nv;
-            for (int j = 0; j < nv; ++j) mult[j] = std::max(mult[j], l2 * (d[j].x * d[j].x + d[j].y * d[j].y));
-        }
         c->cl_lf = new std::vector<double>(nv, 0.0);
         c->cl_lb = new std::vector<double>(nv, 0.0);
         for (int j = 0; j < nv; ++j) {
@@ -2484,8 +2481,9 @@ int vv_create(const vv_grid* grid, vv_ctx** out) {
         const char* ec = getenv("VV_CLUSTER");
         const int ctas = ec && ec[0] ? atoi(ec) : cl_default_ctas(c);
         if (!(sh && sh[0]) && ctas > 0) {
-            const vv::ClShape t = vv::cl_shape(nx, nv, c->pow2, ctas, c->mixed ? 4 : 8, vv::cl_smem_limit(c->mixed));
-            if (t.ctas && vv::cl_resident(c->mixed, t.fam, t.ctas, t.smem) > 0) {
+            const vv::ClShape t = vv::cl_shape(nx, nv, c->pow2, ctas, c->mixed ? 4 : 8,
+                                               vv::cl_smem_limit(c->mixed, vv::cl_family(nx, c->pow2)));
+            if (t.ctas && vv::cl_resident(c->mixed, t.fam, t.ctas) > 0) {
                 s = cl_prepare(c, t);
                 if (s != VV_OK && s != VV_ERR_ALLOC) {
                     vv_destroy(c);
@@ -3693,8 +3691,9 @@ int cl_batch_build(vv_batch* b) {
         vv::ClShape t{};
         if (cl_covers(c))
             for (int ctas = cl_batch_ctas(c); ctas <= vv::CL_MAXC && !t.ctas; ctas *= 2) {
-                t = vv::cl_shape(c->nx, c->nv, c->pow2, ctas, c->mixed ? 4 : 8, vv::cl_smem_limit(c->mixed));
-                if (t.ctas && vv::cl_resident(c->mixed, t.fam, t.ctas, t.smem) < 1) t = vv::ClShape{};
+                t = vv::cl_shape(c->nx, c->nv, c->pow2, ctas, c->mixed ? 4 : 8,
+                                 vv::cl_smem_limit(c->mixed, vv::cl_family(c->nx, c->pow2)));
+                if (t.ctas && vv::cl_resident(c->mixed, t.fam, t.ctas) < 1) t = vv::ClShape{};
             }
         b->cost[i] = (double)c->ncell;
         const int s = t.ctas ? cl_prepare(c, t) : VV_OK;
@@ -3725,6 +3724,7 @@ int cl_batch_build(vv_batch* b) {
     CK(cudaMallocHost((void**)&b->horder, n * sizeof(int)));
     int s = upload_vec(&b->cltab, tab);
     if (s != VV_OK) return s;
+    CK(cudaStreamSynchronize(0));   // the contexts' tables (cl_prepare)
     for (auto& k : b->classes) {
         CK(cudaStreamCreateWithPriority(&k.st, cudaStreamNonBlocking, k.ctas == vv::CL_MAXC ? hi : lo));
         CK(cudaEventCreateWithFlags(&k.done, cudaEventDisableTiming));

@@ -37,27 +37,33 @@ __global__ void k_cl_table(const C* __restrict__ dinv, const C* __restrict__ lam
 
 }  // namespace
 
-size_t cl_smem_limit(bool fp32) {
+int cl_family(int nx, bool pow2) {
+    const int M = nx / 2;
+    return pow2 && M >= 32 && M <= 256 ? M : 0;
+}
+
+// set up for the kernels that are asked for: the attributes load a kernel, which
+// costs milliseconds
+size_t cl_smem_limit(bool fp32, int fam) {
     static std::mutex mu;
-    static size_t limit[64][2] = {};
-    int dev = 0;
+    static size_t limit[64][2][5] = {};
+    int dev = 0, q = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+    for (int m = 32; m <= fam; m *= 2) ++q;
     std::lock_guard<std::mutex> lock(mu);
-    size_t& l = limit[dev][fp32 ? 1 : 0];
+    size_t& l = limit[dev][fp32 ? 1 : 0][q];
     if (l == 0) {
-        int optin = 0, least = 1 << 30;
-        if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) return 0;
-        for (int fam : {0, 32, 64, 128, 256}) {
-            cudaFuncAttributes fa;
-            const void* k = kernel_of(fp32, fam);
-            if (cudaFuncGetAttributes(&fa, k) != cudaSuccess) return 0;
-            const int dyn = optin - (int)fa.sharedSizeBytes;
-            if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn) != cudaSuccess ||
-                cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
-                return 0;
-            least = std::min(least, dyn);
-        }
-        l = (size_t)least;
+        int optin = 0;
+        cudaFuncAttributes fa;
+        const void* k = kernel_of(fp32, fam);
+        if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess ||
+            cudaFuncGetAttributes(&fa, k) != cudaSuccess)
+            return cudaGetLastError(), 0;
+        const int dyn = optin - (int)fa.sharedSizeBytes;
+        if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn) != cudaSuccess ||
+            cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
+            return cudaGetLastError(), 0;
+        l = (size_t)dyn;
     }
     return l;
 }
@@ -65,8 +71,7 @@ size_t cl_smem_limit(bool fp32) {
 ClShape cl_shape(int nx, int nv, bool pow2, int ctas, int tsz, size_t smem_limit) {
     ClShape s{};
     if (nx > CL_NXMAX || ctas < 1 || ctas > CL_MAXC) return s;
-    const int M = nx / 2;
-    s.fam = pow2 && M >= 32 && M <= 256 ? M : 0;
+    s.fam = cl_family(nx, pow2);
     s.slots = cl_slots(s.fam, nx);
     s.rows = (nv + ctas - 1) / ctas;
     // chunks of about eight rows, of at most CL_CHUNK, one thread per (chunk, slot)
@@ -86,13 +91,12 @@ ClShape cl_shape(int nx, int nv, bool pow2, int ctas, int tsz, size_t smem_limit
     return s;
 }
 
-int cl_resident(bool fp32, int fam, int ctas, size_t smem) {
-    if (smem > cl_smem_limit(fp32)) return 0;
-    // the answer of each shape is kept: the query costs about a millisecond
+int cl_resident(bool fp32, int fam, int ctas) {
+    const size_t smem = cl_smem_limit(fp32, fam);
+    if (smem == 0) return 0;
+    // the answer of each kind is kept: the query costs about a millisecond
     struct Key {
-        int dev, fp32, fam, ctas;
-        size_t smem;
-        int n;
+        int dev, fp32, fam, ctas, n;
     };
     static std::mutex mu;
     static std::vector<Key> seen;
@@ -100,7 +104,7 @@ int cl_resident(bool fp32, int fam, int ctas, size_t smem) {
     if (cudaGetDevice(&dev) != cudaSuccess) return 0;
     std::lock_guard<std::mutex> lock(mu);
     for (const Key& k : seen)
-        if (k.dev == dev && k.fp32 == (int)fp32 && k.fam == fam && k.ctas == ctas && k.smem == smem) return k.n;
+        if (k.dev == dev && k.fp32 == (int)fp32 && k.fam == fam && k.ctas == ctas) return k.n;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)ctas);
     cfg.blockDim = dim3(CL_THREADS);
@@ -117,7 +121,7 @@ int cl_resident(bool fp32, int fam, int ctas, size_t smem) {
         cudaGetLastError();
         n = 0;
     }
-    if (seen.size() < 4096) seen.push_back({dev, (int)fp32, fam, ctas, smem, n});
+    seen.push_back({dev, (int)fp32, fam, ctas, n});
     return n;
 }
 
@@ -161,9 +165,7 @@ cudaError_t cl_tables(bool fp32, const ClShape& s, int nv, const void* dinv, con
     else
         k_cl_table<double2><<<g, 256, 0, st>>>((const double2*)dinv, (const double2*)lambda, (double2*)dinv_s,
                                                (double2*)lam_s, s.fam, s.slots, nv, ht);
-    cudaError_t e = cudaGetLastError();
-    const cudaError_t e2 = cudaStreamSynchronize(st);
-    return e == cudaSuccess ? e2 : e;
+    return cudaGetLastError();
 }
 
 cudaError_t cl_launch(bool fp32, int fam, const ClInst* tab, const int* order, int n, int ctas, size_t smem, int mode,
