@@ -1978,7 +1978,6 @@ void cl_describe(const vv_ctx* c, const vv::ClShape& sh, const vv_state* st, vv:
     I->kv = sh.kv;
     I->dsm = sh.dsm;
     I->klev = vv::cl_levels(sh, c->nv, c->cl_lf->data(), c->cl_lb->data(), cl_tol(c));
-    I->restart = c->restart;
     I->ncell = c->ncell;
     I->ht_inv = c->ht_inv;
     I->hv = c->hv;

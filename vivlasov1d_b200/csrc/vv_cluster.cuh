@@ -55,7 +55,6 @@ struct ClInst {
     int nx, nv, fam;               // fam: M = nx/2 for the FFT rows, 0 for the direct DFT
     int rows, nch, klev;           // v rows per CTA, row chunks per mode and CTA, carry levels
     int kv, dsm;                   // basis vectors kept in shared memory; 1: the LU reciprocals too
-    int restart;                   // longest cycle the context's basis holds
     size_t ncell;
     double ht_inv, fscale, hv;     // fscale: f1 (J1, J4) or f2 (J2)
     double cA1, cA2;               // scheme constants (Coef<SCHEME>)

@@ -651,13 +651,12 @@ constexpr int POIS_THREADS = 1024;
 // Single CTA.  Inputs: moment partials (or n directly when part == nullptr).
 // Outputs (each optional): n, u, e, a, phi, h1; scal[0] = ||Poisson residual||_2,
 // scal[1] = sum(phi).
-// psm: the scratch, M + 1 complex, nx (padded to even) and nx + 2 doubles.
-__device__ __forceinline__ void moments_poisson_core(double2* psm, const double* __restrict__ part,
-                                                     const double* __restrict__ n_in, double* __restrict__ n,
-                                                     double* __restrict__ u, double* __restrict__ e,
-                                                     double* __restrict__ a, double* __restrict__ phi,
-                                                     double* __restrict__ h1, double* __restrict__ scal,
-                                                     const PoissonParams& p) {
+__device__ __forceinline__ void moments_poisson_cta(const double* __restrict__ part, const double* __restrict__ n_in,
+                                                    double* __restrict__ n, double* __restrict__ u,
+                                                    double* __restrict__ e, double* __restrict__ a,
+                                                    double* __restrict__ phi, double* __restrict__ h1,
+                                                    double* __restrict__ scal, const PoissonParams& p) {
+    extern __shared__ double2 psm[];
     double2* buf = psm;                                   // M + 1 complex
     double* nn = reinterpret_cast<double*>(psm + p.M + 1);  // nx, padded to an even count
     double* ph = nn + ((p.nx + 1) & ~1);                  // nx + 2; 16-byte aligned (read as double2)
@@ -798,14 +797,6 @@ __device__ __forceinline__ void moments_poisson_core(double2* psm, const double*
         scal[0] = sqrt(r2);
         scal[1] = phisum_s;
     }
-}
-__device__ __forceinline__ void moments_poisson_cta(const double* __restrict__ part, const double* __restrict__ n_in,
-                                                    double* __restrict__ n, double* __restrict__ u,
-                                                    double* __restrict__ e, double* __restrict__ a,
-                                                    double* __restrict__ phi, double* __restrict__ h1,
-                                                    double* __restrict__ scal, const PoissonParams& p) {
-    extern __shared__ double2 psm[];
-    moments_poisson_core(psm, part, n_in, n, u, e, a, phi, h1, scal, p);
 }
 static __global__ void __launch_bounds__(POIS_THREADS)
 k_moments_poisson(const double* __restrict__ part, const double* __restrict__ n_in,
