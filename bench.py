@@ -31,12 +31,18 @@ e2e         : the batched mixed step through Batch.step(host=...), which
               same piece out (the two directions overlap).
 batched_fp64: the same table through the batch in FP64 (ksp_rtol 1e-4): the
               gain of batching alone, apart from the FP32 inner solves.  After
-              the first warm-up step it runs as two tables at once on two
+              the first warm-up step it runs as two batches at once on two
               streams (the eighth of the instances that needed the most GMRES
-              iterations, and the rest), 8% faster than one table in FP64;
-              in mixed precision one table is 3% faster than two.
-step_roofline: algorithmic bytes of the timed steps (from the logged
-              Picard and GMRES counts) over their device time.
+              iterations, and the rest), 2% faster than one in FP64; in mixed
+              precision one batch is 6% faster than two.
+step_roofline: algorithmic bytes of the solver's vectors in the timed steps
+              (from the logged Picard and GMRES counts) over their device
+              time; on clusters they are on-chip traffic, not HBM's.
+roofline    : the kernel the timed steps consist of (k_cl_run), bound by the
+              latency of its dependent stages: the step's arithmetic against
+              the arithmetic peaks, and its counted DRAM bytes.
+lockstep_kernels: kernels of a lockstep table of the same instances, which the
+              timed steps do not launch.
 --impl reference : the CPU restatement of the reference algorithm (the C
               port under oracle/) on the same instances, spread over all host
               threads (each instance single-threaded, as separate runs of a
@@ -162,8 +168,10 @@ def reduce_over_ranks(maxes, sums, device):
 
 
 def step_algorithmic_bytes(specs, reps, mixed, restart=30):
-    """Algorithmic HBM bytes of the timed steps from the logged iteration
-    counts: per instance and step, cells x [N_pic (24 + 16 + 8) + N_gmres
+    """Algorithmic bytes of the solver's vectors in the timed steps from the
+    logged iteration counts, wherever they are served from (an instance on a
+    cluster keeps its vector in shared memory and its basis in shared memory
+    and L2; a lockstep table streams both from HBM): per instance and step, cells x [N_pic (24 + 16 + 8) + N_gmres
     (16 + 48) + sum over Arnoldi steps (16 k + 40)] in FP64 (residual, its
     norm and the moments per Picard pass; Jacobian product and the 3-pass
     preconditioner per GMRES iteration; Gram-Schmidt against the k basis
@@ -183,6 +191,28 @@ def step_algorithmic_bytes(specs, reps, mixed, restart=30):
                     gs += 16 * k + 40
             total += cells * (npic * 48 + inner * (gm * 64 + gs))
     return total
+
+
+# arithmetic peaks (TFLOP/s): FP32 nominal (148 SMs x 128 FMA at 1965 MHz), FP64
+# measured (57 FMA per clock and SM)
+PEAK_F32, PEAK_F64 = 74.4, 33.0
+
+
+def step_algorithmic_flops(specs, reps, restart=30):
+    """(FP32, FP64) operations of the timed mixed steps from the logged counts,
+    per cell: FP64 the residual and the moments of a Picard pass (50 + 6) and
+    Gram-Schmidt against the k basis vectors of the cycle (4 k + 4: the FP32
+    basis is widened); FP32 the Jacobian stencil (28), the FFT pair (5 log2 nx)
+    and the two sweeps of the tridiagonal solve (38 per complex unknown)."""
+    f32 = f64 = 0.0
+    for rep in reps:
+        for s, r in zip(specs, rep):
+            cells = s["nx"] * s["nv"]
+            f64 += cells * 56 * r["picard_its"]
+            for m in r["gmres_its"]:
+                f32 += cells * m * (28 + 5 * np.log2(s["nx"]) + 19)
+                f64 += cells * sum(4 * (it % restart + 1) + 4 for it in range(m))
+    return float(f32), float(f64)
 
 
 def time_steps(fn, k, stream):
@@ -255,9 +285,9 @@ def run_gpu(args, rank, world):
     fe_rel_b64 = np.abs(fe_b - fe_p) / np.abs(fe_p)
     step_bytes = step_algorithmic_bytes(specs, reps, mixed=True)
     step_bytes64 = step_algorithmic_bytes(specs, reps64, mixed=False)
-    # ---- roofline kernels on the whole table (between steps, on the timed
-    # batch itself: the same kernel shapes; the launches overwrite its GMRES
-    # scratch, which every step re-initialises) ----
+    step_flops = step_algorithmic_flops(specs, reps)
+    # ---- the kernels of a lockstep table of the same instances (VV_CLUSTER=0),
+    # between steps; the timed steps launch none of them ----
     mdot_s = batch.time_kernel(0, it=MDOT_IT, reps=20)
     maxpy_s = batch.time_kernel(3, it=MDOT_IT, reps=20)
     pc_s = batch.time_kernel(1, it=MDOT_IT, reps=10)
@@ -288,7 +318,7 @@ def run_gpu(args, rank, world):
                 launches=launches, clocks=clocks, picard=picard, gmres=gmres, fe_rel=fe_rel, fe_rel_b64=fe_rel_b64,
                 fe_m=fe_m, fe_p=fe_p, fe_b=fe_b,
                 mdot_s=mdot_s, maxpy_s=maxpy_s, pc_s=pc_s, jvp_s=jvp_s, tri_s=tri_s, op_s=op_s, mode_rows=mode_rows,
-                step_bytes=step_bytes, step_bytes64=step_bytes64, specs=specs)
+                step_bytes=step_bytes, step_bytes64=step_bytes64, step_flops=step_flops, specs=specs)
 
 
 def port_runs(specs):
@@ -452,9 +482,11 @@ def main():
     b64 = work / res["t_b64"] / 1e9
     peak, peak_kind = measured_peaks()
     step_roofline = {
-        "what": "algorithmic bytes of the whole timed steps (per instance: cells x [N_pic x 48 + N_gmres x 64 + "
-                "sum over Arnoldi steps (16 k + 40)] B in FP64, the FP32 inner terms halved) from the logged "
-                "Picard/GMRES counts, over the device time of the steps",
+        "what": "algorithmic bytes of the solver's vectors in the timed steps (per instance: cells x [N_pic x 48 + "
+                "N_gmres x 64 + sum over Arnoldi steps (16 k + 40)] B in FP64, the FP32 inner terms halved) from the "
+                "logged Picard/GMRES counts, over the device time of the steps.  Not HBM traffic: instances on "
+                "clusters hold these vectors in shared memory and L2; the DRAM bytes counted in one step are under "
+                "roofline.traffic",
         "bytes_per_step": res["step_bytes"] / args.steps,
         "achieved": res["step_bytes"] / res["t_value"] / 1e9, "peak": peak, "unit": "GB/s",
         "frac": res["step_bytes"] / res["t_value"] / 1e9 / peak,
@@ -465,29 +497,43 @@ def main():
     # the tridiagonal stage: read the FP32 complex spectrum and the LU
     # reciprocals, write the solution (3 x 8 B per mode and row)
     tri_bytes = res["mode_rows"] * 24
-    achieved = mdot_bytes / res["mdot_s"] / 1e9
     tri_gbps = tri_bytes / res["tri_s"] / 1e9
-    roofline = {"kernel": "multi-dot of the Gram-Schmidt step (k_b_gm_mdot_p, whole table at Arnoldi index %d; "
-                          "the largest share of the lockstep table's launch list)" % MDOT_IT,
-                "bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                "peak_kind": peak_kind, "traffic": profiled_traffic("batch_mdot_traffic.json"),
-                "algorithmic_bytes_per_launch": mdot_bytes, "avg_launch_us": res["mdot_s"] * 1e6,
-                "others": {"tridiagonal_us": res["tri_s"] * 1e6, "tridiagonal_achieved_GBps": tri_gbps,
-                           "tridiagonal_frac": tri_gbps / peak, "tridiagonal_bytes_per_launch": tri_bytes,
-                           "tridiagonal_traffic": profiled_traffic("batch_tridiag_traffic.json"),
-                           "multiaxpy_us": res["maxpy_s"] * 1e6,
-                           "multiaxpy_achieved_GBps": maxpy_bytes / res["maxpy_s"] / 1e9,
-                           "multiaxpy_frac": maxpy_bytes / res["maxpy_s"] / 1e9 / peak,
-                           "preconditioner_3_kernels_us": res["pc_s"] * 1e6,
-                           "preconditioner_achieved_GBps": cells * 24 / res["pc_s"] / 1e9,
-                           "jacobian_stencil_us": res["jvp_s"] * 1e6,
-                           "jacobian_achieved_GBps": cells * 8 / res["jvp_s"] / 1e9,
-                           # P^-1 J as the step applies it (the stencil fused into the x-FFT when tuned so):
-                           # x read and the result written (4 B each per cell), the half spectrum written
-                           # by the x-FFT and read by the inverse (8 B each per complex unknown), the
-                           # tridiagonal stage (24 B per complex unknown)
-                           "gmres_operator_us": res["op_s"] * 1e6,
-                           "gmres_operator_achieved_GBps": (cells * 8 + res["mode_rows"] * 40) / res["op_s"] / 1e9}}
+    f32, f64 = res["step_flops"]
+    arith_s = f32 / (PEAK_F32 * 1e12) + f64 / (PEAK_F64 * 1e12)
+    # k_cl_run is the whole timed step but for one gather of the reports
+    roofline = {"kernel": "k_cl_run (an instance's whole implicit step on its thread-block cluster; one launch per "
+                          "row length and cluster size, side by side)",
+                "bound": "latency",
+                "note": "chains of dependent stages between cluster barriers, one 512-thread CTA per SM: issue slots "
+                        "25-40% busy, DRAM idle (profiles/cluster_step.md); achieved and peak in the mix of the "
+                        "step's FP32 and FP64 operations",
+                "achieved": (f32 + f64) / res["t_value"] / 1e12, "peak": (f32 + f64) / arith_s / 1e12,
+                "unit": "TFLOP/s", "frac": arith_s / res["t_value"],
+                "peak_kind": "FP32 nominal %.1f, FP64 measured %.1f TFLOP/s" % (PEAK_F32, PEAK_F64),
+                "traffic": profiled_traffic("cluster_step_traffic.json")}
+    lockstep = {"path": "a lockstep table of the same instances (VV_CLUSTER=0 or VV_BATCH_SHAPE); not launched by the "
+                        "timed steps",
+                "peak": peak, "peak_kind": peak_kind, "unit": "GB/s",
+                "multidot": {"kernel": "k_b_gm_mdot_p, Arnoldi index %d" % MDOT_IT, "bound": "hbm",
+                             "achieved": mdot_bytes / res["mdot_s"] / 1e9, "frac": mdot_bytes / res["mdot_s"] / 1e9 / peak,
+                             "traffic": profiled_traffic("batch_mdot_traffic.json"),
+                             "algorithmic_bytes_per_launch": mdot_bytes, "avg_launch_us": res["mdot_s"] * 1e6},
+                "tridiagonal_us": res["tri_s"] * 1e6, "tridiagonal_achieved_GBps": tri_gbps,
+                "tridiagonal_frac": tri_gbps / peak, "tridiagonal_bytes_per_launch": tri_bytes,
+                "tridiagonal_traffic": profiled_traffic("batch_tridiag_traffic.json"),
+                "multiaxpy_us": res["maxpy_s"] * 1e6,
+                "multiaxpy_achieved_GBps": maxpy_bytes / res["maxpy_s"] / 1e9,
+                "multiaxpy_frac": maxpy_bytes / res["maxpy_s"] / 1e9 / peak,
+                "preconditioner_3_kernels_us": res["pc_s"] * 1e6,
+                "preconditioner_achieved_GBps": cells * 24 / res["pc_s"] / 1e9,
+                "jacobian_stencil_us": res["jvp_s"] * 1e6,
+                "jacobian_achieved_GBps": cells * 8 / res["jvp_s"] / 1e9,
+                # P^-1 J as the table applies it (the stencil fused into the x-FFT when tuned so):
+                # x read and the result written (4 B each per cell), the half spectrum written
+                # by the x-FFT and read by the inverse (8 B each per complex unknown), the
+                # tridiagonal stage (24 B per complex unknown)
+                "gmres_operator_us": res["op_s"] * 1e6,
+                "gmres_operator_achieved_GBps": (cells * 8 + res["mode_rows"] * 40) / res["op_s"] / 1e9}
     fe = res["fe_rel"]
     cpu = None
     fe_err = {"steps": args.warmup + args.steps, "max": float(fe.max()), "median": float(np.median(fe)),
@@ -522,7 +568,7 @@ def main():
             "step_roofline": step_roofline,
             "field_energy_rel_err": fe_err,
             "e2e": {"value": e2e, "unit": METRIC, "h2d_bytes_per_step": cells * 8, "d2h_bytes_per_step": cells * 8},
-            "gpu_launches": res["launches"], "roofline": roofline, "clocks": res["clocks"],
+            "gpu_launches": res["launches"], "roofline": roofline, "lockstep_kernels": lockstep, "clocks": res["clocks"],
             "iterations": {"picard_per_step_mean": res["picard"], "gmres_per_step_mean": res["gmres"]}}
     if cpu is not None:
         line["cpu_baseline"] = cpu
