@@ -18,9 +18,11 @@ re-forms it as two tables -- the eighth of the instances that needed the
 most GMRES iterations, and the rest -- which every later step launches at
 once on two streams (``vv_batch_launch``) and collects together
 (``vv_batch_collect``), so that the two tables' passes interleave.  Instances
-on clusters do not wait for one another and gain nothing by it.  Each instance computes the same
-operations in either form (the tables' tuned kernel shapes may differ, so
-results agree to rounding).
+on clusters do not wait for one another: a batch of clusters gains little by
+it (256-instance sweep in FP64, where the largest instances form a table:
+34.1 -> 33.4 ms a step) or loses (mixed precision, all on clusters: 18.7 ->
+20.0 ms).  Each instance computes the same operations in either form (the
+tables' tuned kernel shapes may differ, so results agree to rounding).
 
 The host stands between two steps: ``step()`` waits for the step's
 reports before it returns, and the next step's graph starts when the host
