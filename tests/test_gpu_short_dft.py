@@ -1,6 +1,7 @@
 """The direct DFT of short rows (one tile of 32 modes, a warp per row) and just
-beyond it, row blocks part full: along x in the kinetic preconditioner, along
-the field's columns in the potential one, and in FP32 inside a mixed step."""
+beyond it, in length and (FP64, 1600 rows) in number, row blocks part full:
+along x in the kinetic preconditioner, along the field's columns in the
+potential one, and in FP32 inside a mixed step."""
 import numpy as np
 import pytest
 
@@ -17,7 +18,7 @@ def _cuda():
 
 
 @pytest.mark.parametrize("nx,nv", [(5, 13), (6, 16), (17, 18), (31, 17), (33, 50), (61, 12), (62, 15), (63, 33),
-                                   (65, 14), (66, 9)])
+                                   (65, 14), (66, 9), (55, 1601), (57, 1601), (59, 1599)])
 def test_short_rows_match_oracle(nx, nv):
     """1e-12 (kinetic) and 1e-11 (potential) relative, as every variant of the preconditioners."""
     from vivlasov1d_b200.solver import Grid, TensorProductPreconditioner

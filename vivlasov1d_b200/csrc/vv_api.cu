@@ -517,13 +517,32 @@ size_t rdft_smem(int nx, size_t csz) {
 }
 size_t irdft_smem(int nx, size_t csz) { return rdft_smem(nx, csz); }
 
+// the direct DFT of p.nv rows of p.nx values (COLS: of the columns of a field `cols` wide)
+template <typename TI, typename R, bool COLS>
+void launch_rdft(vv_ctx* c, const TI* X, typename Cplx<R>::type* spec, const vv::PcParams& p, int cols) {
+    auto blocks = [&](int rows) { return (unsigned)((p.nv + rows - 1) / rows); };
+    if (vv::dft_is_short(p.nx, p.nv, std::is_same<R, double>::value))
+        vv::k_rdft_short<TI, R, COLS><<<blocks(vv::DFT_SHORT_ROWS), vv::DFT_SHORT_THREADS, 0, c->st>>>(X, spec, p, cols);
+    else
+        vv::k_rdft_rows<TI, R, COLS><<<blocks(vv::DFT_ROWS), vv::DFT_THREADS,
+                                       rdft_smem(p.nx, sizeof(typename Cplx<R>::type)), c->st>>>(X, spec, p, cols);
+}
+template <typename R, typename TO, bool COLS>
+void launch_irdft(vv_ctx* c, const typename Cplx<R>::type* spec, TO* Y, const vv::PcParams& p, int cols) {
+    auto blocks = [&](int rows) { return (unsigned)((p.nv + rows - 1) / rows); };
+    if (vv::dft_is_short(p.nx, p.nv, std::is_same<R, double>::value))
+        vv::k_irdft_short<R, TO, COLS><<<blocks(vv::DFT_SHORT_ROWS), vv::DFT_SHORT_THREADS, 0, c->st>>>(spec, Y, p, cols);
+    else
+        vv::k_irdft_rows<R, TO, COLS><<<blocks(vv::DFT_ROWS), vv::DFT_THREADS,
+                                        irdft_smem(p.nx, sizeof(typename Cplx<R>::type)), c->st>>>(spec, Y, p, cols);
+}
+
 template <typename TI, typename R>
 int launch_rfft(vv_ctx* c, const TI* X, typename Cplx<R>::type* spec, const vv::PcParams& p, unsigned rows) {
     const size_t csz = sizeof(typename Cplx<R>::type);
     const int M = c->M;
     if (c->fft_kind == 2 || !c->pow2) {
-        const unsigned g = (unsigned)((c->nv + vv::DFT_ROWS - 1) / vv::DFT_ROWS);
-        vv::k_rdft_rows<TI, R><<<g, vv::DFT_THREADS, rdft_smem(c->nx, csz), c->st>>>(X, spec, p, 0);
+        launch_rdft<TI, R, false>(c, X, spec, p, 0);
     } else if (c->fft_kind == 1 && four_step_ok(M)) {
         const size_t sm = fft_smem(1, M, c->pcR, csz, false);
         switch (M / 32) {
@@ -545,8 +564,7 @@ int launch_irfft(vv_ctx* c, const typename Cplx<R>::type* spec, TO* Y, const vv:
     const size_t csz = sizeof(typename Cplx<R>::type);
     const int M = c->M;
     if (c->fft_kind == 2 || !c->pow2) {
-        const unsigned g = (unsigned)((c->nv + vv::DFT_ROWS - 1) / vv::DFT_ROWS);
-        vv::k_irdft_rows<R, TO><<<g, vv::DFT_THREADS, irdft_smem(c->nx, csz), c->st>>>(spec, Y, p, 0);
+        launch_irdft<R, TO, false>(c, spec, Y, p, 0);
     } else if (c->fft_kind == 1 && four_step_ok(M)) {
         const size_t sm = fft_smem(1, M, c->pcR, csz, true);
         switch (M / 32) {
@@ -934,9 +952,9 @@ int pcv_apply_t(vv_ctx* c, const TI* X, TO* Y, const int* yidx = nullptr, int yo
     p.yoff = 0;
     p.ystride = 0;
     const size_t csz = sizeof(C2);
-    const unsigned gr = (unsigned)((nx + c->pvR - 1) / c->pvR), gd = (unsigned)((nx + vv::DFT_ROWS - 1) / vv::DFT_ROWS);
+    const unsigned gr = (unsigned)((nx + c->pvR - 1) / c->pvR);
     if (fft) vv::k_rfft_rows<R, R><<<gr, 32 * c->pvR, fft_smem(0, nv / 2, c->pvR, csz, false), c->st>>>(xt, spec, p);
-    else vv::k_rdft_rows<TI, R, true><<<gd, vv::DFT_THREADS, rdft_smem(nv, csz), c->st>>>(X, spec, p, nx);   // rows = the field's columns
+    else launch_rdft<TI, R, true>(c, X, spec, p, nx);   // rows = the field's columns
     CKL(c);
     const vv::PotLu<C2>& lu = [&]() -> const vv::PotLu<C2>& {
         if constexpr (D) return c->pv_lu;
@@ -954,7 +972,7 @@ int pcv_apply_t(vv_ctx* c, const TI* X, TO* Y, const int* yidx = nullptr, int yo
         p.yidx = yidx;
         p.yoff = yoff;
         p.ystride = yidx ? c->ncell : 0;
-        vv::k_irdft_rows<R, TO, true><<<gd, vv::DFT_THREADS, irdft_smem(nv, csz), c->st>>>(spec, Y, p, nx);
+        launch_irdft<R, TO, true>(c, spec, Y, p, nx);
         CKL(c);
         return VV_OK;
     }

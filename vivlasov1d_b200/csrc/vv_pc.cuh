@@ -423,10 +423,7 @@ __global__ void k_irfft4(const typename Cplx<R>::type* __restrict__ spec, TO* __
 // sum and difference are staged).  With fewer than eight tiles of modes the
 // sum over n is split over the warps.  201 x 401 in FP64: forward 8.5 us,
 // inverse 9.2 us, the function call that holds them 49 -> 28.7 us.
-// With one tile (nx < 64) a warp takes one row instead: there the split's
-// barrier and sums cost more than the few products it spreads (whole FP64
-// preconditioner, 152 v rows: nx 17 9.26 -> 7.8 us, nx 56 9.99 -> 9.2; each
-// row's sum halved over two warps: 8.0 and 9.3).
+// Rows of one tile (nx < 64): the short kernels below.
 // ---------------------------------------------------------------------------
 constexpr int DFT_ROWS = 4, DFT_THREADS = 256, DFT_WARPS = DFT_THREADS / 32;
 
@@ -457,24 +454,6 @@ VV_DEV void dft_join(C (&v)[DFT_ROWS], const DftSplit& s, C* red) {
 #pragma unroll
             for (int r = 0; r < DFT_ROWS; ++r)
                 v[r] = c_add(v[r], red[(((q - 1) * s.nT + s.tile) * DFT_ROWS + r) * 32 + lane]);
-    }
-}
-
-// v_r += sum over [na, nb) of (Re x Re w, Im x Im w), w = W^{n kk}, x row r's entry n (RW rows)
-template <int RW, typename C>
-VV_DEV void dft_sums(C (&v)[RW], const C* xs, int nm, const C* stw, int N, int kk, int na, int nb) {
-    int idx = kk * na % N;
-#pragma unroll 2
-    for (int n = na; n < nb; ++n) {
-        const C w = stw[idx];
-#pragma unroll
-        for (int r = 0; r < RW; ++r) {
-            const C x = xs[r * nm + n];
-            v[r].x += x.x * w.x;
-            v[r].y += x.y * w.y;
-        }
-        idx += kk;
-        if (idx >= N) idx -= N;
     }
 }
 
@@ -515,15 +494,6 @@ k_rdft_rows(const TI* __restrict__ X, typename Cplx<R>::type* __restrict__ spec,
         xs[r * nm + n] = v;
     }
     __syncthreads();
-    if (nm <= 32) {   // one tile: a warp one row
-        const int r = threadIdx.x >> 5, k = threadIdx.x & 31, kk = k < nm ? k : 0;
-        if (r >= DFT_ROWS || j0 + r >= p.nv) return;
-        const C e = xs[r * nm];
-        C v[1] = {c_make<C>((double)(e.x + ((kk & 1) ? -e.y : e.y)), 0.0)};
-        dft_sums(v, xs + r * nm, nm, stw, N, kk, 1, half + 1);
-        if (k < nm) spec[(size_t)k * p.nv + j0 + r] = v[0];
-        return;
-    }
     const DftSplit s(nm);
     for (int tile = s.tile; tile < s.nT; tile += s.step) {
         const int k = tile * 32 + (threadIdx.x & 31), kk = k < nm ? k : 0;
@@ -536,7 +506,19 @@ k_rdft_rows(const TI* __restrict__ X, typename Cplx<R>::type* __restrict__ spec,
         }
         if (s.part < s.parts) {
             const int na = 1 + s.part * half / s.parts, nb = 1 + (s.part + 1) * half / s.parts;
-            dft_sums(v, xs, nm, stw, N, kk, na, nb);
+            int idx = (int)((long long)kk * na % N);
+#pragma unroll 2
+            for (int n = na; n < nb; ++n) {
+                const C w = stw[idx];
+#pragma unroll
+                for (int r = 0; r < DFT_ROWS; ++r) {
+                    const C x = xs[r * nm + n];
+                    v[r].x += x.x * w.x;
+                    v[r].y += x.y * w.y;
+                }
+                idx += kk;
+                if (idx >= N) idx -= N;
+            }
         }
         dft_join(v, s, red);
         if (s.part == 0 && k < nm) {
@@ -568,24 +550,6 @@ k_irdft_rows(const typename Cplx<R>::type* __restrict__ spec, TO* __restrict__ Y
     }
     __syncthreads();
     const R inv = (R)(1.0 / (double)N);
-    // samples n and N - n of row r from the sums t
-    auto put = [&](int r, int n, C t) {
-        const C* xr = xs + r * nm;
-        R e = xr[0].x;
-        if (!(N & 1)) e += (n & 1) ? -xr[N / 2].x : xr[N / 2].x;
-        TO* row = Y + (COLS ? (size_t)(j0 + r) : (size_t)(j0 + r) * N);
-        const size_t es = COLS ? (size_t)cols : 1;
-        row[n * es] = (TO)((e + (R)2 * (t.x + t.y)) * inv);
-        if (n > 0 && 2 * n != N) row[(N - n) * es] = (TO)((e + (R)2 * (t.x - t.y)) * inv);
-    };
-    if (nm <= 32) {
-        const int r = threadIdx.x >> 5, n = threadIdx.x & 31;
-        if (r >= DFT_ROWS || j0 + r >= p.nv) return;
-        C v[1] = {c_make<C>(0.0, 0.0)};
-        dft_sums(v, xs + r * nm, nm, stw, N, n < nm ? n : 0, 1, K + 1);
-        if (n < nm) put(r, n, v[0]);
-        return;
-    }
     const DftSplit s(nm);
     for (int tile = s.tile; tile < s.nT; tile += s.step) {
         const int n = tile * 32 + (threadIdx.x & 31), nn = n < nm ? n : 0;
@@ -593,17 +557,124 @@ k_irdft_rows(const typename Cplx<R>::type* __restrict__ spec, TO* __restrict__ Y
 #pragma unroll
         for (int r = 0; r < DFT_ROWS; ++r) v[r].x = v[r].y = R(0);
         if (s.part < s.parts) {
-            // W^{nk} = (cos, -sin): Re(X e^{+i theta}) = X.x w.x + X.y w.y
             const int ka = 1 + s.part * K / s.parts, kb = 1 + (s.part + 1) * K / s.parts;
-            dft_sums(v, xs, nm, stw, N, nn, ka, kb);
+            int idx = (int)((long long)nn * ka % N);
+#pragma unroll 2
+            for (int k = ka; k < kb; ++k) {
+                const C w = stw[idx];   // W^{nk} = (cos, -sin): Re(X e^{+i theta}) = X.x w.x + X.y w.y
+#pragma unroll
+                for (int r = 0; r < DFT_ROWS; ++r) {
+                    const C x = xs[r * nm + k];
+                    v[r].x += x.x * w.x;
+                    v[r].y += x.y * w.y;
+                }
+                idx += nn;
+                if (idx >= N) idx -= N;
+            }
         }
         dft_join(v, s, red);
         if (s.part == 0 && n < nm) {
 #pragma unroll
             for (int r = 0; r < DFT_ROWS; ++r)
-                if (j0 + r < p.nv) put(r, n, v[r]);
+                if (j0 + r < p.nv) {
+                    const C* xr = xs + r * nm;
+                    R e = xr[0].x;
+                    if (!(N & 1)) e += (n & 1) ? -xr[N / 2].x : xr[N / 2].x;
+                    TO* row = Y + (COLS ? (size_t)(j0 + r) : (size_t)(j0 + r) * N);
+                    const size_t es = COLS ? (size_t)cols : 1;
+                    row[n * es] = (TO)((e + (R)2 * (v[r].x + v[r].y)) * inv);
+                    if (n > 0 && 2 * n != N) row[(N - n) * es] = (TO)((e + (R)2 * (v[r].x - v[r].y)) * inv);
+                }
         }
     }
+}
+
+// Short rows (nx/2 + 1 <= 32, one tile of modes): a warp one row, a lane one mode
+// (sample), the row and the twiddles in shared memory.  Spreading such a sum over
+// warps costs more in the join's barrier than the few products it spreads; and
+// as a branch of the kernels above it cost them registers (72 instead of 64:
+// three blocks an SM instead of four).  Whole FP64 preconditioner, with the split
+// -> here: 17 x 152 9.3 -> 7.7 us, 50 x 152 9.9 -> 9.1, 17 x 2048 15.9 -> 12.8.
+constexpr int DFT_SHORT = 32, DFT_SHORT_ROWS = 4, DFT_SHORT_THREADS = 32 * DFT_SHORT_ROWS;
+// Many FP64 rows of almost a tile are better off above, where a gathered twiddle
+// serves four rows: 61 x 1531 15.2 there and 15.1 us here, 61 x 1813 17.0 and 17.5,
+// 50 x 2048 17.1 and 16.6; in FP32 61 x 2048 14.7 and 13.2.
+inline bool dft_is_short(int nx, int rows, bool fp64) {
+    const int nm = nx / 2 + 1;
+    return nm <= DFT_SHORT && !(fp64 && nm > 28 && rows > 1600);
+}
+template <typename C> struct DftShort {   // shared memory of a block
+    C tw[2 * DFT_SHORT], x[DFT_SHORT_ROWS][DFT_SHORT];
+};
+// sums over n = 1..half of (Re x Re w, Im x Im w), w = W^{n kk}
+template <typename C> VV_DEV C dft_short_sums(C v, const C* x, const C* tw, int N, int kk, int half) {
+    int idx = 0;
+#pragma unroll 2
+    for (int n = 1; n <= half; ++n) {
+        idx += kk;
+        if (idx >= N) idx -= N;
+        const C w = tw[idx], e = x[n];
+        v.x += e.x * w.x;
+        v.y += e.y * w.y;
+    }
+    return v;
+}
+
+template <typename TI, typename R, bool COLS = false>
+__global__ void __launch_bounds__(DFT_SHORT_THREADS)
+k_rdft_short(const TI* __restrict__ X, typename Cplx<R>::type* __restrict__ spec, PcParams p, int cols) {
+    using C = typename Cplx<R>::type;
+    __shared__ DftShort<C> sm;
+    const int N = p.nx, nm = N / 2 + 1, half = (N - 1) / 2, j0 = blockIdx.x * DFT_SHORT_ROWS;
+    const C* tw = reinterpret_cast<const C*>(p.tw);
+    for (int k = threadIdx.x; k < N; k += DFT_SHORT_THREADS) sm.tw[k] = tw[k];
+    for (int i = threadIdx.x; i < DFT_SHORT_ROWS * DFT_SHORT; i += DFT_SHORT_THREADS) {
+        const int r = COLS ? i % DFT_SHORT_ROWS : i / DFT_SHORT, n = COLS ? i / DFT_SHORT_ROWS : i % DFT_SHORT;
+        if (n > half || j0 + r >= p.nv) continue;
+        const TI* row = X + (COLS ? (size_t)(j0 + r) : (size_t)(j0 + r) * N);
+        const size_t es = COLS ? (size_t)cols : 1;
+        const R a = (R)row[n * es], b = n > 0 ? (R)row[(N - n) * es] : (N & 1) ? R(0) : (R)row[(N / 2) * es];
+        C v;   // (x_0, x_{N/2} or 0), then (x_n + x_{N-n}, x_n - x_{N-n})
+        v.x = n > 0 ? a + b : a;
+        v.y = n > 0 ? a - b : b;
+        sm.x[r][n] = v;
+    }
+    __syncthreads();
+    const int r = threadIdx.x >> 5, k = threadIdx.x & 31;
+    if (k >= nm || j0 + r >= p.nv) return;
+    const C e = sm.x[r][0];
+    C v;
+    v.x = e.x + ((k & 1) ? -e.y : e.y);
+    v.y = R(0);
+    spec[(size_t)k * p.nv + j0 + r] = dft_short_sums(v, sm.x[r], sm.tw, N, k, half);
+}
+
+template <typename R, typename TO, bool COLS = false>
+__global__ void __launch_bounds__(DFT_SHORT_THREADS)
+k_irdft_short(const typename Cplx<R>::type* __restrict__ spec, TO* __restrict__ Y, PcParams p, int cols) {
+    using C = typename Cplx<R>::type;
+    if (p.yidx) Y += (size_t)(*p.yidx + p.yoff) * p.ystride;
+    __shared__ DftShort<C> sm;
+    const int N = p.nx, nm = N / 2 + 1, half = (N - 1) / 2, j0 = blockIdx.x * DFT_SHORT_ROWS;
+    const C* tw = reinterpret_cast<const C*>(p.tw);
+    for (int k = threadIdx.x; k < N; k += DFT_SHORT_THREADS) sm.tw[k] = tw[k];
+    for (int i = threadIdx.x; i < DFT_SHORT_ROWS * nm; i += DFT_SHORT_THREADS) {
+        const int r = i % DFT_SHORT_ROWS, k = i / DFT_SHORT_ROWS;
+        if (j0 + r < p.nv) sm.x[r][k] = spec[(size_t)k * p.nv + j0 + r];
+    }
+    __syncthreads();
+    const int r = threadIdx.x >> 5, n = threadIdx.x & 31;
+    if (n >= nm || j0 + r >= p.nv) return;
+    C v;
+    v.x = v.y = R(0);
+    v = dft_short_sums(v, sm.x[r], sm.tw, N, n, half);
+    R e = sm.x[r][0].x;
+    if (!(N & 1)) e += (n & 1) ? -sm.x[r][N / 2].x : sm.x[r][N / 2].x;
+    const R inv = (R)(1.0 / (double)N);
+    TO* row = Y + (COLS ? (size_t)(j0 + r) : (size_t)(j0 + r) * N);
+    const size_t es = COLS ? (size_t)cols : 1;
+    row[n * es] = (TO)((e + (R)2 * (v.x + v.y)) * inv);
+    if (n > 0 && 2 * n != N) row[(N - n) * es] = (TO)((e + (R)2 * (v.x - v.y)) * inv);
 }
 
 // ---------------------------------------------------------------------------
