@@ -1965,13 +1965,17 @@ int step_host(vv_ctx* c, vv_state* st) {
 // path, which the tests compare with).  Sixteen wherever the instance fits:
 // two steps of 64 x 256 in FP64 take 498 us on 16 CTAs, 524 on 8, 622 on 4
 // and 1417 in the multi-kernel graph; 256 x 512, the largest that fits in
-// FP64, 1670 against 2240.  The direct-DFT rows cost rows nx^2 per CTA and
-// lose from about a million on (300 x 100, 0.63 M: 1.9x faster; 200 x 400,
-// 1.0 M: even; 201 x 401, 1.05 M: 7% slower).
+// FP64, 1670 against 2240.  The direct-DFT rows cost rows nx^2 per CTA on 16
+// of the SMs: the line is where two steps and a linear solve take as long on
+// the multi-kernel path (on the cluster / off it, us, FP64 steps: 75 x 1021
+// 1836 / 2037, 75 x 1533 2478 / 2155, 100 x 765 1514 / 1600, 100 x 1021 1823 /
+// 1705, 150 x 381 1837 / 1814, 250 x 189 2239 / 2274, 300 x 189 3084 / 2879;
+// mixed 75 x 1533 2376 / 2654, 100 x 1021 1866 / 1918, 100 x 1533 2621 / 2145).
 int cl_default_ctas(const vv_ctx* c) {
-    const int rows = (c->nv + vv::CL_MAXC - 1) / vv::CL_MAXC;
+    const double rows = (c->nv + vv::CL_MAXC - 1) / vv::CL_MAXC, nx = c->nx;
     const bool dft = !(c->pow2 && c->nx >= 64);
-    return dft && (double)rows * c->nx * c->nx > 9e5 ? 0 : vv::CL_MAXC;
+    const double line = c->mixed ? 3.5e5 + 3100 * nx : 2.5e5 + 2000 * nx;
+    return dft && rows * nx * nx > std::min(9e5, line) ? 0 : vv::CL_MAXC;
 }
 
 // configurations the cluster kernel covers: the factored Arakawa brackets with
